@@ -61,6 +61,15 @@ __device__ __forceinline__ unsigned long long ld_volatile_u64(const void *p) {
 	asm volatile("ld.volatile.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
 	return v;
 }
+// the same from shared or global memory
+__device__ __forceinline__ unsigned long long ld_volatile_generic_u64(const void *p) {
+	unsigned long long v;
+	asm volatile("ld.volatile.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+	return v;
+}
+__device__ __forceinline__ void st_volatile_shared_f64(double *p, double v) {
+	asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "d"(v) : "memory");
+}
 __device__ __forceinline__ void st_volatile_f64(double *p, double v) {
 	asm volatile("st.volatile.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
@@ -230,7 +239,8 @@ struct bsg_fct {
 	double *d_ur_v, *d_lr_v;      // FP64 strict values
 	float *d_ur_f, *d_lr_f;       // FP32 strict values
 	int nnz_strict;
-	int *d_perm;                  // rows by (forward-solve level, index): claim order of the solves
+	int *d_perm;                  // exact solves: rows by (block, forward-solve level, index)
+	int trsv_rows;                // consecutive rows a block
 	bsg_sell sl, su;              // SELL-32 strict L / U rows (Jacobi sweeps), FP64 or FP32
 	int levels_l, levels_u;       // dependency depth
 	double density, density2;
@@ -273,6 +283,7 @@ int bsg_trisolve_launch(bsg_ctx *c, const bsg_fct *f, int lower, int mode, int n
 // the two-sided Lanczos; builds the transposed forms on first use.
 int bsg_trisolve_t_launch(bsg_ctx *c, bsg_fct *f, int which, int mode, int nsweeps, const double *x, double *y,
                           double *work);
+int bsg_trsv_schedule(bsg_ctx *c, bsg_fct *f, const int *lev);
 int bsg_check_devstat(bsg_ctx *c);
 // block ILU2 / IC2 of a 3x3 block matrix (k_bfact.cu) and its solves
 int bsg_bfact_run(bsg_ctx *c, bsg_mat *m, int sym, const bsg_param *p, bsg_fct **out);

@@ -50,7 +50,6 @@
 #include "bsg_internal.cuh"
 #include "bsg_blk3.cuh"
 #include <cub/device/device_scan.cuh>
-#include <cub/device/device_radix_sort.cuh>
 
 #define F_U 0u
 #define F_R 1u
@@ -1580,13 +1579,6 @@ __global__ void k_emit_u(int n, int kind, const unsigned long long *rec, const u
 	}
 }
 
-__global__ void k_level_keys(int n, const int *lev, unsigned long long *keys, int *vals) {
-	int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	keys[i] = ((unsigned long long)(unsigned)lev[i] << 32) | (unsigned)i;
-	vals[i] = i;
-}
-
 // block rows: stored blocks per row, then the rows in order (pivot scaling
 // first: column i; U blocks +column, R blocks -column), counts of U / R
 __global__ void k_blk_len(int nb, const unsigned long long *rec, int *cnt) {
@@ -1699,8 +1691,8 @@ int bsg_fact_run(bsg_ctx *c, bsg_mat *m, int kind, const bsg_param *p, bsg_fct *
 	BSG_CUDA(cudaMemsetAsync(c->d_stat, 0, sizeof(bsg_devstat), st));
 
 	cudaEventRecord(c->ev0, st);
-	// scale, init, queue fill, seed, rows, count, emit, level keys (+ CUB scans/sorts)
-	BSG_COUNT(8);
+	// scale, init, queue fill, seed, rows, count, emit (+ CUB scans)
+	BSG_COUNT(7);
 	k_fact_scale<<<nb(n, 256), 256, 0, st>>>(n, kind, m->d_iu, m->d_ju, m->d_al, p->sclmin, scll, sclu, diag0, c->d_stat);
 	k_fact_init<<<nb(n, 256), 256, 0, st>>>(n, m->d_it, nstat, whead, rec, acc, lev, inprog, c->d_stat);
 	k_fill_int<<<BSG_SMS * 4, 256, 0, st>>>(qcap, queue, -1);
@@ -1787,25 +1779,10 @@ int bsg_fact_run(bsg_ctx *c, bsg_mat *m, int kind, const bsg_param *p, bsg_fct *
 	BSG_CUDA(cudaMallocAsync(&f->d_u, sizeof(double) * nzu, st));
 	k_emit_u<<<nb(n, 256), 256, 0, st>>>(n, kind, rec, cf, pl, pu, scll, sclu, iu, f->d_ju, f->d_l, f->d_u);
 	BSG_CUDA(cudaGetLastError());
-	// level schedule of the triangular solves: rows by (forward level, index)
-	{
-		unsigned long long *keys, *k2;
-		int *vals;
-		BSG_CUDA(cudaMallocAsync(&keys, sizeof(unsigned long long) * n, st));
-		BSG_CUDA(cudaMallocAsync(&k2, sizeof(unsigned long long) * n, st));
-		BSG_CUDA(cudaMallocAsync(&vals, sizeof(int) * n, st));
-		BSG_CUDA(cudaMallocAsync(&f->d_perm, sizeof(int) * n, st));
-		k_level_keys<<<nb(n, 256), 256, 0, st>>>(n, lev, keys, vals);
-		size_t t2 = 0;
-		BSG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t2, keys, k2, vals, f->d_perm, n, 0, 64, st));
-		void *d_t2;
-		BSG_CUDA(cudaMallocAsync(&d_t2, t2 > 0 ? t2 : 1, st));
-		BSG_CUDA(cub::DeviceRadixSort::SortPairs(d_t2, t2, keys, k2, vals, f->d_perm, n, 0, 64, st));
-		unsigned long long last = 0;
-		if (n > 0) BSG_CUDA(cudaMemcpyAsync(&last, k2 + n - 1, sizeof(last), cudaMemcpyDeviceToHost, st));
-		BSG_CUDA(cudaStreamSynchronize(st));
-		f->levels_l = f->levels_u = n > 0 ? (int)(last >> 32) + 1 : 0;
-		cudaFreeAsync(keys, st); cudaFreeAsync(vals, st); cudaFreeAsync(k2, st); cudaFreeAsync(d_t2, st);
+	rc = bsg_trsv_schedule(c, f, lev);
+	if (rc) {
+		release();
+		return rc;
 	}
 	cudaEventRecord(c->ev1, st);
 	f->density = (double)nzu / (double)m->nnz_up;

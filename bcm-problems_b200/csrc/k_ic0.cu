@@ -116,13 +116,6 @@ __global__ void k_ic0_scatter_off(int nk, const int *lpos, const double *lv, dou
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t < nk) u[lpos[t]] = lv[t];
 }
-__global__ void k_ic0_level_keys(int n, const int *lev, unsigned long long *keys, int *vals) {
-	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	keys[i] = ((unsigned long long)(unsigned)lev[i] << 32) | (unsigned)i;
-	vals[i] = i;
-}
-
 struct Dev {
 	void *p = nullptr;
 	cudaStream_t s = nullptr;
@@ -141,8 +134,8 @@ int bsg_ic0_run(bsg_ctx *c, bsg_mat *m, bsg_fct **out) {
 	cudaEventRecord(c->ev0, s);
 	int rc = bsg_strict_transpose(c, n, m->d_iu, m->d_ju, nnz, &it, &jt, &lpos, &nk);
 	if (rc) return rc;
-	Dev dit, djt, dlp, dlv, ddinv, dlev, ddone, dclaim, dkeys, dk2, dvals, dtmp;
-	for (Dev *d : {&dit, &djt, &dlp, &dlv, &ddinv, &dlev, &ddone, &dclaim, &dkeys, &dk2, &dvals, &dtmp}) d->s = s;
+	Dev dit, djt, dlp, dlv, ddinv, dlev, ddone, dclaim;
+	for (Dev *d : {&dit, &djt, &dlp, &dlv, &ddinv, &dlev, &ddone, &dclaim}) d->s = s;
 	dit.p = it;
 	djt.p = jt;
 	dlp.p = lpos;
@@ -172,39 +165,17 @@ int bsg_ic0_run(bsg_ctx *c, bsg_mat *m, bsg_fct **out) {
 	rc = BSG_OK;
 	if (cudaMallocAsync(&f->d_iu, sizeof(int) * (n + 1), s) != cudaSuccess ||
 	    cudaMallocAsync(&f->d_ju, sizeof(int) * (nnz > 0 ? nnz : 1), s) != cudaSuccess ||
-	    cudaMallocAsync(&f->d_u, sizeof(double) * (nnz > 0 ? nnz : 1), s) != cudaSuccess ||
-	    cudaMallocAsync(&f->d_perm, sizeof(int) * (n > 0 ? n : 1), s) != cudaSuccess)
+	    cudaMallocAsync(&f->d_u, sizeof(double) * (nnz > 0 ? nnz : 1), s) != cudaSuccess)
 		rc = bsg_set_error(BSG_ERR_NOMEM, "IC(0) factor");
 	if (!rc) {
 		f->d_l = f->d_u;
 		cudaMemcpyAsync(f->d_iu, m->d_iu, sizeof(int) * (n + 1), cudaMemcpyDeviceToDevice, s);
 		cudaMemcpyAsync(f->d_ju, m->d_ju, sizeof(int) * nnz, cudaMemcpyDeviceToDevice, s);
-		BSG_COUNT(3);
+		BSG_COUNT(2);
 		k_ic0_scatter_diag<<<nb(n, 256), 256, 0, s>>>(n, m->d_iu, (double *)ddinv.p, f->d_u);
 		k_ic0_scatter_off<<<nb(nk, 256), 256, 0, s>>>(nk, lpos, (double *)dlv.p, f->d_u);
-		// the level schedule of the triangular solves: rows by (depth, index)
-		if (cudaMallocAsync(&dkeys.p, sizeof(unsigned long long) * (n > 0 ? n : 1), s) != cudaSuccess ||
-		    cudaMallocAsync(&dk2.p, sizeof(unsigned long long) * (n > 0 ? n : 1), s) != cudaSuccess ||
-		    cudaMallocAsync(&dvals.p, sizeof(int) * (n > 0 ? n : 1), s) != cudaSuccess)
-			rc = bsg_set_error(BSG_ERR_NOMEM, "IC(0) level schedule");
 	}
-	if (!rc) {
-		k_ic0_level_keys<<<nb(n, 256), 256, 0, s>>>(n, (int *)dlev.p, (unsigned long long *)dkeys.p, (int *)dvals.p);
-		size_t tb = 0;
-		cub::DeviceRadixSort::SortPairs(nullptr, tb, (unsigned long long *)dkeys.p, (unsigned long long *)dk2.p,
-		                                (int *)dvals.p, f->d_perm, n, 0, 64, s);
-		if (cudaMallocAsync(&dtmp.p, tb > 0 ? tb : 1, s) != cudaSuccess) rc = bsg_set_error(BSG_ERR_NOMEM, "IC(0) sort");
-		if (!rc && cub::DeviceRadixSort::SortPairs(dtmp.p, tb, (unsigned long long *)dkeys.p, (unsigned long long *)dk2.p,
-		                                           (int *)dvals.p, f->d_perm, n, 0, 64, s) != cudaSuccess)
-			rc = bsg_set_error(BSG_ERR_CUDA, "IC(0) sort");
-	}
-	if (!rc) {
-		unsigned long long last = 0;
-		if (n > 0)
-			cudaMemcpyAsync(&last, (unsigned long long *)dk2.p + (n - 1), sizeof(last), cudaMemcpyDeviceToHost, s);
-		if (cudaStreamSynchronize(s) != cudaSuccess) rc = bsg_set_error(BSG_ERR_CUDA, "IC(0)");
-		f->levels_l = f->levels_u = n > 0 ? (int)(last >> 32) + 1 : 0;
-	}
+	if (!rc) rc = bsg_trsv_schedule(c, f, (int *)dlev.p);
 	cudaEventRecord(c->ev1, s);
 	if (!rc) rc = bsg_fct_finish(c, f);
 	if (rc) {

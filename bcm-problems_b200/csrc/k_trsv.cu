@@ -7,12 +7,11 @@
 //   forward  y_i = dinv_l[i] * (x_i - sum_{k<i} L(i,k) y_k)
 //   backward y_i = dinv_u[i] * (x_i - sum_{k>i} U(i,k) y_k)
 //
-// mode 0 -- exact, sync-free: a warp solves one row; warps claim rows in
-//   dependency order (ascending for L, descending for U) from an atomic
-//   counter, and each lane waits on the entry it needs.  "Solved" is encoded
-//   in the value itself: y is pre-filled with a NaN bit pattern no arithmetic
-//   produces, and a 64-bit store publishes the result in one transaction.
-//   Every wait is bounded by globaltimer (BSG_ERR_TIMEOUT).
+// mode 0 -- exact, sync-free: a warp solves one row, in level order within the
+//   block of consecutive rows its CTA owns, and each lane waits on the entry it
+//   needs.  "Solved" is encoded in the value itself: y is pre-filled with a NaN
+//   bit pattern no arithmetic produces, and a 64-bit store publishes the result
+//   in one transaction.  Every wait is bounded by globaltimer (BSG_ERR_TIMEOUT).
 // mode 1 -- Jacobi sweeps: y <- D^{-1}(x - N y) repeated nsweeps times from
 //   y = D^{-1} x; every sweep is a fully parallel pass over the factor (HBM
 //   bound: 4 B value (FP32) or 8 B (FP64) + 4 B column per entry).  It applies
@@ -20,6 +19,7 @@
 //   preconditioner and, applied symmetrically, a valid PCG preconditioner.
 #include "bsg_internal.cuh"
 #include "k_stream.cuh"
+#include <cub/device/device_radix_sort.cuh>
 
 #ifndef SELL_SIGMA
 #define SELL_SIGMA 128 // rows per length-sorting window of the factor's sliced copies
@@ -44,48 +44,219 @@ __global__ void k_scale_vec(int n, const double *x, const double *d, double *y) 
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) y[i] = x[i] * d[i];
 }
 
-// Rows are claimed in the order of `perm` (ascending forward-solve level;
-// read backwards for U), a topological order of both dependency graphs that
-// keeps the rows in flight on the current wavefront.
+// ---- exact solve ------------------------------------------------------------
+// Bound: the longest chain of dependent rows times the latency of one link, so
+// the kernel is laid out for short links.
+//  - Every CTA owns a block of consecutive rows and solves them in level order,
+//    its warps taking the rows in turn.  In natural order most dependencies lie
+//    close by, so most links stay inside a CTA and pass through shared memory
+//    (ys); only links between blocks go through L2.
+//  - A row's columns, values, right-hand side and inverse pivot are in registers
+//    before its wait; the next row's load during it.
+//  - With one entry of the row still unsolved, the warp has already added up
+//    the rest: the waiting lane holds the five partial sums that the butterfly
+//    of warp_sum() would add to its own and adds them in that order, so the
+//    result has the bits of the plain reduction, without its shuffles after
+//    the wait.
+// All CTAs must be resident (a cooperative launch): the unsolved row that comes
+// first by (level, place in its list) depends on solved rows only, and its warp
+// has no earlier row left, so the solve always progresses.
+// Measured against one warp per row claimed in global level order with every
+// link through L2 (us per forward solve, before / after, FP64 IC2 tau 1e-3 of the
+// 7-point heat operator): 12^3 553 / 145, 32^3 1668 / 309, 47x40x33 3537 / 514,
+// 128^3 18690 / 5470; IC(0) 128^3 2075 / 1170; 2-D 500^2 22752 / 1836; a chain of
+// 100000 rows 437 / 21 ms (0.21 us a link).  A random graph with 30 levels has
+// no links to keep inside a block: 249 / 285.
+#define TRSV_WARPS 32 // 24 warps: 47x40x33 580, 128^3 5520; 16: 760, 6600 // entries of a row each lane holds (32 TRSV_M a row; longer rows walk their head first)
+#define TRSV_ROWS_MAX 28000 // rows of a block: 8 bytes each in shared memory
+// fewest rows of a block: smaller blocks spread a small system over more SMs,
+// larger ones keep more links inside (us, 12^3 / 47x40x33: 128 rows 144 / 521,
+// 256 146 / 516, 512 152 / 566, 1024 158 / 634)
+#define TRSV_ROWS_MIN 256
+
+// The solved entry at p (shared or global), waiting for it; the spin limit or
+// another warp's failure gives 0.
+__device__ __forceinline__ unsigned long long trsv_wait(const double *p, int row, bsg_devstat *st) {
+	unsigned long long raw = ld_volatile_generic_u64(p);
+	if (raw != BSG_PENDING) return raw;
+	unsigned long long t0 = 0;
+	for (unsigned it = 1;; it++) {
+		raw = ld_volatile_generic_u64(p);
+		if (raw != BSG_PENDING) return raw;
+		if ((it & 127) == 0) {
+			if (*(volatile int *)&st->code != 0) return 0;
+			const unsigned long long now = globaltimer_ns();
+			if (t0 == 0) t0 = now;
+			else if (now - t0 > BSG_SPIN_LIMIT_NS) {
+				devstat_fail(st, BSG_ERR_TIMEOUT, row);
+				return 0;
+			}
+		}
+	}
+}
+
 template <typename VT>
-__global__ void __launch_bounds__(256) k_trsv_syncfree(int n, int lower, const int *__restrict__ perm,
-                                                       const int *__restrict__ rp, const int *__restrict__ ci,
-                                                       const VT *__restrict__ v, int skip_first,
-                                                       const double *__restrict__ dinv, const double *__restrict__ x,
-                                                       double *y, unsigned *claim, bsg_devstat *st) {
-	const int lane = threadIdx.x & 31;
-	for (;;) {
-		int t = 0;
-		if (lane == 0) t = (int)atomicAdd(claim, 1u);
-		t = __shfl_sync(0xffffffffu, t, 0);
-		if (t >= n) return;
-		const int row = perm[lower ? t : n - 1 - t];
-		const int b = rp[row] + skip_first, e = rp[row + 1];
-		double s = 0.0;
-		for (int k = b + lane; k < e; k += 32) {
-			const int c = ci[k];
-			unsigned long long raw = ld_volatile_u64(y + c);
-			if (raw == BSG_PENDING) {
-				unsigned long long t0 = globaltimer_ns();
-				for (unsigned it = 1;; it++) {
-					__nanosleep(32);
-					raw = ld_volatile_u64(y + c);
-					if (raw != BSG_PENDING) break;
-					if ((it & 127) == 0) {
-						if (*(volatile int *)&st->code != 0) { raw = 0; break; }
-						if (globaltimer_ns() - t0 > BSG_SPIN_LIMIT_NS) {
-							devstat_fail(st, BSG_ERR_TIMEOUT, row);
-							raw = 0;
-							break;
-						}
+__global__ void __launch_bounds__(TRSV_WARPS * 32, 1)
+k_trsv_blocks(int n, int lower, int block0, int rows, const int *__restrict__ perm, const int *__restrict__ rp,
+              const int *__restrict__ ci, const VT *__restrict__ v, int skip_first, const double *__restrict__ dinv,
+              const double *__restrict__ x, double *y, bsg_devstat *st) {
+	extern __shared__ double ys[]; // the block's solved rows, BSG_PENDING before
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int r0 = (block0 + blockIdx.x) * rows, cnt = min(rows, n - r0);
+	// item k of this warp: place warp + k TRSV_WARPS of the block's list (read backwards for U)
+	auto item = [&](int k) {
+		const int o = warp + k * TRSV_WARPS;
+		return o < cnt ? perm[r0 + (lower ? o : cnt - 1 - o)] : -1;
+	};
+	struct Meta {
+		int row, b, e;
+		double x, d;
+	};
+	auto meta = [&](int row) {
+		Meta m = {row, 0, 0, 0.0, 0.0};
+		if (row >= 0) {
+			m.b = rp[row] + skip_first;
+			m.e = rp[row + 1];
+			m.x = x[row];
+			m.d = dinv[row];
+		}
+		return m;
+	};
+	int row1 = item(lane);
+	for (int k = threadIdx.x; k < cnt; k += blockDim.x) ys[k] = __longlong_as_double((long long)BSG_PENDING);
+	Meta cur = meta(row1);
+	row1 = item(32 + lane);
+	__syncthreads();
+	int nc[TRSV_M];
+	VT nv[TRSV_M];
+	auto load = [&](int b, int e) { // the last 32 TRSV_M entries of a row at most
+		const int tail = max(b, b + ((e - b - 1) / 32 - (TRSV_M - 1)) * 32);
+#pragma unroll
+		for (int u = 0; u < TRSV_M; u++) {
+			const int k = tail + u * 32 + lane;
+			nc[u] = -1;
+			nv[u] = VT(0);
+			if (k < e) {
+				nc[u] = ci[k];
+				nv[u] = v[k];
+			}
+		}
+	};
+	load(__shfl_sync(0xffffffffu, cur.b, 0), __shfl_sync(0xffffffffu, cur.e, 0));
+	for (int k0 = 0; warp + k0 * TRSV_WARPS < cnt; k0 += 32) {
+		const Meta nxt = meta(row1); // 32 rows ahead
+		row1 = item(k0 + 64 + lane);
+		for (int j = 0; j < 32 && warp + (k0 + j) * TRSV_WARPS < cnt; j++) {
+			const int row = __shfl_sync(0xffffffffu, cur.row, j);
+			const int b = __shfl_sync(0xffffffffu, cur.b, j), e = __shfl_sync(0xffffffffu, cur.e, j);
+			const double xr = __shfl_sync(0xffffffffu, cur.x, j), dr = __shfl_sync(0xffffffffu, cur.d, j);
+			int c[TRSV_M];
+			double a[TRSV_M];
+#pragma unroll
+			for (int u = 0; u < TRSV_M; u++) {
+				c[u] = nc[u];
+				a[u] = (double)nv[u];
+			}
+			load(__shfl_sync(0xffffffffu, j < 31 ? cur.b : nxt.b, (j + 1) & 31),
+			     __shfl_sync(0xffffffffu, j < 31 ? cur.e : nxt.e, (j + 1) & 31));
+			auto entry = [&](int col) -> const double * {
+				const unsigned s = (unsigned)(col - r0);
+				return s < (unsigned)cnt ? ys + s : y + col;
+			};
+			double s = 0.0;
+			if (e - b > 32 * TRSV_M) { // head of a long row, in order
+				const int tail = b + ((e - b - 1) / 32 - (TRSV_M - 1)) * 32;
+				for (int k = b + lane; k < tail; k += 32) {
+					const int col = ci[k];
+					s = fma((double)v[k], __longlong_as_double((long long)trsv_wait(entry(col), row, st)), s);
+				}
+				__syncwarp();
+			}
+			const double *src[TRSV_M];
+			unsigned long long raw[TRSV_M];
+#pragma unroll
+			for (int u = 0; u < TRSV_M; u++) {
+				src[u] = c[u] >= 0 ? entry(c[u]) : nullptr;
+				raw[u] = src[u] ? BSG_PENDING : 0ull;
+			}
+			// poll until at most one lane waits
+			unsigned wait;
+			unsigned long long t0 = 0;
+			for (unsigned it = 1;; it++) {
+				bool mine = false;
+#pragma unroll
+				for (int u = 0; u < TRSV_M; u++) {
+					if (raw[u] == BSG_PENDING) raw[u] = ld_volatile_generic_u64(src[u]);
+					mine = mine || raw[u] == BSG_PENDING;
+				}
+				wait = __ballot_sync(0xffffffffu, mine);
+				if ((wait & (wait - 1)) == 0) break;
+				if ((it & 127) == 0) { // the limit, or another warp's failure: leave the rest at 0
+					bool give = *(volatile int *)&st->code != 0;
+					const unsigned long long now = globaltimer_ns();
+					if (t0 == 0) t0 = now;
+					else if (!give && now - t0 > BSG_SPIN_LIMIT_NS) {
+						devstat_fail(st, BSG_ERR_TIMEOUT, row);
+						give = true;
+					}
+					if (__any_sync(0xffffffffu, give)) {
+#pragma unroll
+						for (int u = 0; u < TRSV_M; u++)
+							if (raw[u] == BSG_PENDING) raw[u] = 0;
+						wait = 0;
+						break;
 					}
 				}
 			}
-			s = fma((double)v[k], __longlong_as_double((long long)raw), s);
+			const int last = wait ? __ffs(wait) - 1 : 0; // the lane that finishes the row
+			double t = s;
+			if (wait == 0 || lane != last) {
+#pragma unroll
+				for (int u = 0; u < TRSV_M; u++)
+					if (c[u] >= 0) t = fma(a[u], __longlong_as_double((long long)raw[u]), t);
+			}
+			double part[5];
+			{
+				double r = t;
+#pragma unroll
+				for (int k = 0; k < 5; k++) {
+					part[k] = __shfl_xor_sync(0xffffffffu, r, 16 >> k);
+					r += part[k];
+				}
+			}
+			if (lane == last) {
+				if (wait) {
+#pragma unroll
+					for (int u = 0; u < TRSV_M; u++)
+						if (c[u] >= 0) {
+							if (raw[u] == BSG_PENDING) raw[u] = trsv_wait(src[u], row, st);
+							t = fma(a[u], __longlong_as_double((long long)raw[u]), t);
+						}
+				}
+#pragma unroll
+				for (int k = 0; k < 5; k++) t += part[k];
+				const double yr = (xr - t) * dr;
+				st_volatile_shared_f64(ys + (row - r0), yr);
+				st_volatile_f64(y + row, yr);
+			}
+			__syncwarp();
 		}
-		s = warp_sum(s);
-		if (lane == 0) st_volatile_f64(y + row, (x[row] - s) * dinv[row]);
+		cur = nxt;
 	}
+}
+
+// Sort keys of the solve order: the row's block, then its level; *most gets the
+// largest level.
+__global__ void k_trsv_keys(int n, int rows, const int *lev, unsigned long long *keys, int *vals) {
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= n) return;
+	keys[i] = ((unsigned long long)(unsigned)(i / rows) << 32) | (unsigned)lev[i];
+	vals[i] = i;
+}
+__global__ void k_trsv_levels(int n, const int *lev, int *most) {
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	const int m = __reduce_max_sync(0xffffffffu, i < n ? lev[i] : 0);
+	if ((threadIdx.x & 31) == 0) atomicMax(most, m);
 }
 
 template <int G, typename VT>
@@ -110,6 +281,7 @@ __global__ void __launch_bounds__(256) k_trsv_jacobi(int n, const int *__restric
 	}
 }
 
+// y before an exact solve: nothing solved
 __global__ void k_fill_u64(long long n, unsigned long long *p, unsigned long long v) {
 	for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
 		p[i] = v;
@@ -139,7 +311,49 @@ inline int nb(long long n, int t) { return n > 0 ? (int)((n + t - 1) / t) : 1; }
 
 int bsg_strict_transpose(bsg_ctx *c, int n, const int *ia, const int *ja, int nnz, int **it_o, int **jt_o,
                          int **perm_o, int *nnz_o);
-int bsg_choose_group(double mean_row);
+
+// The exact solves' order of f's n rows from their levels (ascending depth in
+// the forward solve's dependency graph): blocks of f->trsv_rows consecutive
+// rows, by (level, index) inside a block, in f->d_perm; sets levels_l / levels_u.
+int bsg_trsv_schedule(bsg_ctx *c, bsg_fct *f, const int *lev) {
+	cudaStream_t s = c->stream;
+	const int n = f->n;
+	f->levels_l = f->levels_u = 0;
+	f->trsv_rows = TRSV_ROWS_MIN;
+	BSG_CUDA(cudaMallocAsync(&f->d_perm, sizeof(int) * (n > 0 ? n : 1), s));
+	if (n <= 0) return BSG_OK;
+	// an equal share per SM, but no less than TRSV_ROWS_MIN (a smaller block has
+	// more of its links outside) and no more than shared memory holds
+	long long rows = (n + BSG_SMS - 1) / BSG_SMS;
+	if (rows < TRSV_ROWS_MIN) rows = TRSV_ROWS_MIN;
+	if (rows > TRSV_ROWS_MAX) {
+		const long long steps = (n + (long long)BSG_SMS * TRSV_ROWS_MAX - 1) / ((long long)BSG_SMS * TRSV_ROWS_MAX);
+		rows = (n + steps * BSG_SMS - 1) / (steps * BSG_SMS);
+	}
+	f->trsv_rows = (int)rows;
+	int bits = 32;
+	while ((1ll << (bits - 32)) < (n + rows - 1) / rows) bits++;
+	unsigned long long *keys = nullptr, *k2 = nullptr;
+	int *vals = nullptr, *most = nullptr, top = 0;
+	void *tmp = nullptr;
+	size_t tb = 0;
+	BSG_CUDA(cudaMallocAsync(&keys, sizeof(unsigned long long) * n, s));
+	BSG_CUDA(cudaMallocAsync(&k2, sizeof(unsigned long long) * n, s));
+	BSG_CUDA(cudaMallocAsync(&vals, sizeof(int) * n, s));
+	BSG_CUDA(cudaMallocAsync(&most, sizeof(int), s));
+	BSG_CUDA(cudaMemsetAsync(most, 0, sizeof(int), s));
+	BSG_COUNT(2);
+	k_trsv_levels<<<nb(n, 256), 256, 0, s>>>(n, lev, most);
+	k_trsv_keys<<<nb(n, 256), 256, 0, s>>>(n, f->trsv_rows, lev, keys, vals);
+	BSG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
+	BSG_CUDA(cudaMallocAsync(&tmp, tb > 0 ? tb : 1, s));
+	BSG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
+	BSG_CUDA(cudaMemcpyAsync(&top, most, sizeof(int), cudaMemcpyDeviceToHost, s));
+	BSG_CUDA(cudaStreamSynchronize(s));
+	f->levels_l = f->levels_u = top + 1;
+	for (void *q : {(void *)keys, (void *)k2, (void *)vals, (void *)most, tmp}) cudaFreeAsync(q, s);
+	return BSG_OK;
+}
 
 // Build the gather forms of a freshly compacted factor.
 int bsg_fct_finish(bsg_ctx *c, bsg_fct *f) {
@@ -229,19 +443,40 @@ int trisolve_impl(bsg_ctx *c, const bsg_fct *f, const TriOp &t, int mode, int ns
 	const int n = f->n;
 	const bool use32 = f->fp32 != 0;
 	if (mode == 0) {
-		BSG_COUNT(2); // fill + solve
-		k_fill_u64<<<BSG_SMS * 4, 256, 0, s>>>(n, (unsigned long long *)y, BSG_PENDING);
-		unsigned *claim = c->d_counters + 1;
-		BSG_CUDA(cudaMemsetAsync(claim, 0, sizeof(unsigned), s));
-		int grid = BSG_SMS * 8;
-		int need = (n + 7) / 8;
-		if (grid > need) grid = need > 0 ? need : 1;
-		if (use32)
-			k_trsv_syncfree<float><<<grid, 256, 0, s>>>(n, t.lower, f->d_perm, t.rp, t.ci, t.vf, t.skip, t.dinv, x, y, claim,
-			                                           c->d_stat);
-		else
-			k_trsv_syncfree<double><<<grid, 256, 0, s>>>(n, t.lower, f->d_perm, t.rp, t.ci, t.vd, t.skip, t.dinv, x, y,
-			                                            claim, c->d_stat);
+		BSG_COUNT(1);
+		const int fill = nb(n, 256) < BSG_SMS * 4 ? nb(n, 256) : BSG_SMS * 4;
+		k_fill_u64<<<fill, 256, 0, s>>>(n, (unsigned long long *)y, BSG_PENDING);
+		const int rows = f->trsv_rows, blocks = n > 0 ? (n + rows - 1) / rows : 0;
+		// at most one block per SM at a time: larger systems take several
+		// launches over consecutive blocks, in solve order
+		const int steps = (blocks + BSG_SMS - 1) / BSG_SMS;
+		for (int k = 0; k < steps; k++) {
+			const int b0 = (t.lower ? k : steps - 1 - k) * BSG_SMS;
+			cudaLaunchConfig_t cfg = {};
+			cfg.gridDim = dim3(blocks - b0 < BSG_SMS ? blocks - b0 : BSG_SMS);
+			cfg.blockDim = dim3(TRSV_WARPS * 32);
+			cfg.dynamicSmemBytes = sizeof(double) * rows;
+			cfg.stream = s;
+			cudaLaunchAttribute coop;
+			coop.id = cudaLaunchAttributeCooperative;
+			coop.val.cooperative = 1;
+			cfg.attrs = &coop;
+			cfg.numAttrs = 1;
+			BSG_COUNT(1);
+			cudaError_t e;
+			if (use32) {
+				cudaFuncSetAttribute(k_trsv_blocks<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				                     (int)sizeof(double) * TRSV_ROWS_MAX);
+				e = cudaLaunchKernelEx(&cfg, k_trsv_blocks<float>, n, t.lower, b0, rows, (const int *)f->d_perm, t.rp, t.ci,
+				                       t.vf, t.skip, t.dinv, x, y, c->d_stat);
+			} else {
+				cudaFuncSetAttribute(k_trsv_blocks<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				                     (int)sizeof(double) * TRSV_ROWS_MAX);
+				e = cudaLaunchKernelEx(&cfg, k_trsv_blocks<double>, n, t.lower, b0, rows, (const int *)f->d_perm, t.rp, t.ci,
+				                       t.vd, t.skip, t.dinv, x, y, c->d_stat);
+			}
+			BSG_CUDA(e);
+		}
 		return cudaGetLastError() == cudaSuccess ? BSG_OK : BSG_ERR_CUDA;
 	}
 	if (nsweeps < 1) nsweeps = 1;
