@@ -144,3 +144,73 @@ def test_unet_forward_tensor_core_level_matches_oracle(ctx, ny, nz):
     assert np.all(np.isfinite(got))
     assert np.abs(got - want).max() <= 1e-2 * np.abs(want).max()
     assert np.linalg.norm(got - want) <= 5e-3 * np.linalg.norm(want)
+
+
+def _backward_rounded(A, W, gy):
+    """U.backward with the GPU's storage: every activation gradient in bf16."""
+    q = U.bf16
+    g = q(gy[..., None] * W["w7"] * (A["d0"] > 0))
+    G = {"W6": U.conv_wgrad(A["in6"], g)}
+    gi6 = U.conv_dgrad(g, W["W6"])
+    g = q(U.up_t(gi6[..., :16]) * (A["d1"] > 0))
+    G["W5"] = U.conv_wgrad(A["in5"], g)
+    gi5 = U.conv_dgrad(g, W["W5"])
+    g = q(U.up_t(gi5[..., :32]) * (A["d2"] > 0))
+    G["W4"] = U.conv_wgrad(A["in4"], g)
+    gi4 = U.conv_dgrad(g, W["W4"])
+    g = q(U.up_t(gi4[..., :64]) * (A["e3"] > 0))
+    G["W3"] = U.conv_wgrad(A["p3"], g)
+    g = q((gi4[..., 64:] + U.pool_t(U.conv_dgrad(g, W["W3"]))) * (A["e2"] > 0))
+    G["W2"] = U.conv_wgrad(A["p2"], g)
+    g = q((gi5[..., 32:] + U.pool_t(U.conv_dgrad(g, W["W2"]))) * (A["e1"] > 0))
+    G["W1"] = U.conv_wgrad(A["p1"], g)
+    g = q((gi6[..., 16:] + U.pool_t(U.conv_dgrad(g, W["W1"]))) * (A["e0"] > 0))
+    G["W0"] = U.conv_wgrad(A["x0"], g)
+    return G
+
+
+def _sparse_case(nx, ny, nz):
+    """Weights of +-1 in three places per output channel, an input of 0, +-1/4
+    and +-1: every forward sum is exact in FP32, so the GPU's activations (and the
+    masks of the backward pass) are the reference's."""
+    n = nx * ny * nz
+    rng = np.random.default_rng(n)
+    W = {}
+    for k in U.NAMES:
+        cin, cout = U.CH[k]
+        W[k] = np.zeros((27, cout, cin))
+        for co in range(cout):
+            for t, ci in zip(rng.integers(0, 27, 3), rng.integers(0, 2 if k == "W0" else cin, 3)):
+                W[k][t, co, ci] = rng.choice([1.0, 1.0, -1.0])
+    W["w7"] = rng.choice([1.0, -1.0, 0.5], 16)
+    r = np.zeros(n)
+    r[rng.choice(n, 16, replace=False)] = rng.choice([1.0, -1.0], 16)  # norm 4
+    up = np.zeros(n, bool)
+    up[rng.choice(n, n // 2, replace=False)] = True
+    t = rng.standard_normal(n)
+    logd = np.where(up, 1.0, -1.0).reshape(nz, ny, nx)
+    x0, _ = U.make_input(r.reshape(nz, ny, nx), logd)
+    A = U.forward(x0, W)
+    want = _backward_rounded(A, W, U.loss(A["y"], t.reshape(nz, ny, nx))[1])
+    return W, r, t, np.where(up, np.exp(1.0), np.exp(-1.0)), A, want
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(8, 8, 8), (24, 16, 40), (64, 8, 16), (16, 24, 8)])
+def test_unet_gradients_on_ragged_grids(ctx, nx, ny, nz):
+    """Weight gradients where the bricks of the gradient kernel (8 x 8 x 4
+    voxels) stand over the grid's edges at one level or another, down to a
+    single voxel.  With exact activations and the GPU's bf16 storage in the
+    reference, what is left is FP32 sums and the few gradients they push over a
+    rounding boundary: below one bf16 step of every value, 2^-8."""
+    import bsg
+    import torch
+    W, r, t, d, _, want = _sparse_case(nx, ny, nz)
+    net = bsg.UNet(ctx, nx, ny, nz, train=True)
+    net.set_weights(_flat(W))
+    net.set_diag(torch.as_tensor(d, device="cuda"))
+    net.train_sample(torch.as_tensor(r, device="cuda"), torch.as_tensor(t, device="cuda"))
+    G = _unflat(net.grads())
+    for k in want:
+        err = np.linalg.norm(G[k] - want[k])
+        assert err <= 2.0 ** -8 * np.linalg.norm(want[k]), (k, err)
+    net.free()
