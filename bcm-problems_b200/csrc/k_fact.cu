@@ -14,8 +14,8 @@
 // between m and i", and a member that does not store i has dropped it.
 //
 // Schedule (dynamic, deadlock-free).  A row enters a global FIFO queue when
-// every row of A's column i has been claimed by a warp (a counter per row,
-// decremented when such a row is first claimed).  A warp pops a row and tries it: it builds C(i) over
+// every row of A's column i has been claimed by a warp and all but one or two
+// are finished (see Admission).  A warp pops a row and tries it: it builds C(i) over
 // finished rows (one member per lane, rows read with 16-byte loads).  An
 // unfinished member m that another warp is computing is waited for; a member
 // nobody is computing parks the row on m's waiter list and the warp moves on;
@@ -124,6 +124,7 @@ struct FactArgs {
 	unsigned char *big_ws;     // BIG_SLOTS workspaces of GlobWS<>::bytes
 	int *big_owner;            // 1 while a warp holds that workspace
 	int *nhold;                // warps holding their row for a member nobody computes
+	int *nbig;                 // workspaces taken
 	int hold_max;              // at most this many (half the warps)
 };
 
@@ -140,7 +141,7 @@ struct PhaseClock {
 // a row whose member set, mask or a contributor segment does not fit is
 // tried again by the same warp in a larger workspace in global memory
 // (GlobWS), so any row up to the big capacities factors.  Both expose the
-// same members; sc[] = {members, mask columns, kept columns, blocking row}.
+// same members; sc[0] is the number of members.
 // IC2 (ILU false) keeps one value per column: its shared workspace has no
 // U-side arrays, so more warps fit on an SM.  Block rows (BLK) keep 9
 // values per column (U side; ILU: then the L side at 9 (hcap + slot)) in hl
@@ -178,7 +179,8 @@ struct SmemWS {
 	};
 	double pf_l[BLK ? 1 : PFCAP], pf_u[ILU && !BLK ? PFCAP : 1];
 	int sc[4];
-	int slots[1];          // (the global workspace lists its slots; this one scans them)
+	short slots[hcap];     // the accumulator slots in use, in insertion order (the diagonal first)
+	short srt[hcap];       // the off-diagonal ones among them by ascending column (see sort_columns)
 };
 
 template <bool ILU, bool BLK = false>
@@ -190,11 +192,11 @@ struct GlobWS {
 	static constexpr size_t bytes = 8 * (nval + (size_t)HCAP_BIG + 2 * (size_t)PFCAP_BIG) +
 	                                4 * (7 * (size_t)CMAX_BIG + (CMAX_BIG + 4) + 2 * (size_t)CMAX_BIG +
 	                                     4 * (size_t)HCAP_BIG + PFCAP_BIG + 4) +
-	                                2 * (size_t)PFCAP_BIG + 3 * (size_t)CMAX_BIG + mwin / 8 + 4 * (size_t)HCAP_BIG;
+	                                2 * (size_t)PFCAP_BIG + 3 * (size_t)CMAX_BIG + mwin / 8 + 8 * (size_t)HCAP_BIG;
 	double *hl, *hu, *pf_l, *pf_u;
 	int *W, *Wp, *We, *Ws, *Wps, *Wes, *Wlv, *Wb, *wset, *hkey, *lst, *lsts, *lkey, *sc;
 	unsigned *pf_cf, *wbits;
-	int *slots;            // the accumulator slots in use, in insertion order
+	int *slots, *srt;      // as above
 	short *pf_slot;
 	unsigned char *Wf, *Wfs, *Wst;
 	__device__ explicit GlobWS(unsigned char *p) {
@@ -209,7 +211,7 @@ struct GlobWS {
 		pf_slot = reinterpret_cast<short *>(sc + 4);
 		Wf = reinterpret_cast<unsigned char *>(pf_slot + PFCAP_BIG); Wfs = Wf + CMAX_BIG; Wst = Wfs + CMAX_BIG;
 		wbits = reinterpret_cast<unsigned *>(Wst + CMAX_BIG);
-		slots = reinterpret_cast<int *>(wbits + mwin / 32);
+		slots = reinterpret_cast<int *>(wbits + mwin / 32); srt = slots + HCAP_BIG;
 	}
 };
 
@@ -237,17 +239,20 @@ __device__ __forceinline__ int seg_owner(const int *b, int n, int k) {
 	return lo;
 }
 
-// Find or insert column c; returns slot or -1 if full.
+// Find or insert column c; returns slot or -1 if full.  A lane whose column
+// was new gets fresh set; note_slots then lists the new slots.
 template <class WS>
-__device__ int hfind_insert(WS &s, int c) {
+__device__ int hfind_insert(WS &s, int c, bool &fresh) {
+	fresh = false;
 	unsigned h = hash_u(c) & (s.hcap - 1);
+#pragma unroll 1
 	for (int probe = 0; probe < s.hcap; probe++) {
 		int k = s.hkey[h];
 		if (k == c) return (int)h;
 		if (k == -1) {
 			int old = atomicCAS(&s.hkey[h], -1, c);
 			if (old == -1) {
-				if (WS::big) s.slots[atomicAdd(&s.sc[3], 1)] = (int)h;
+				fresh = true;
 				if (WS::blk) {
 #pragma unroll
 					for (int k = 0; k < 9; k++) s.hl[9 * h + k] = 0.0;
@@ -267,18 +272,22 @@ __device__ int hfind_insert(WS &s, int c) {
 	return -1;
 }
 
+// Append the slots of the lanes with `fresh` to the row's list of ncol slots
+// (the whole warp).
+template <class WS>
+__device__ __forceinline__ void note_slots(WS &s, int &ncol, bool fresh, int h, int lane) {
+	const unsigned b = __ballot_sync(0xffffffffu, fresh);
+	if (fresh) s.slots[ncol + __popc(b & ((1u << lane) - 1))] = h;
+	ncol += __popc(b);
+}
+
 // Insert row k into the member set of row i; 1 if new, 0 if present, -1
 // if full.  Near rows: one bit each.  Far rows: a hash; most candidates are
 // already members, so probe with plain reads and CAS only into an empty slot.
 template <class WS>
-__device__ int wset_insert(WS &s, int i, int k) {
-	const int d = i - 1 - k;
-	if (d < WS::mwin) {
-		const unsigned bit = 1u << (d & 31);
-		if (s.wbits[d >> 5] & bit) return 0;
-		return (atomicOr(&s.wbits[d >> 5], bit) & bit) ? 0 : 1;
-	}
+__device__ int wset_far(WS &s, int k) {
 	unsigned h = hash_u(k) & (s.wcap - 1);
+#pragma unroll 1
 	for (int probe = 0; probe < s.wcap; probe++) {
 		int cur = s.wset[h];
 		if (cur == k) return 0;
@@ -291,11 +300,19 @@ __device__ int wset_insert(WS &s, int i, int k) {
 	}
 	return -1;
 }
+template <class WS>
+__device__ int wset_insert(WS &s, int i, int k) {
+	const int d = i - 1 - k;
+	if (d >= WS::mwin) return wset_far(s, k);
+	const unsigned bit = 1u << (d & 31);
+	if (s.wbits[d >> 5] & bit) return 0;
+	return (atomicOr(&s.wbits[d >> 5], bit) & bit) ? 0 : 1;
+}
 
 // Ranks of keys t0 + 32 q + lane (q < NQ) among the nl distinct keys, by one
 // broadcast key per step; entry t goes to position rank(t) of out.
-template <int NQ>
-__device__ __forceinline__ void rank_sort(const int *key_of, const int *val, int *out, int nl, int t0, int lane) {
+template <int NQ, class OUT>
+__device__ __forceinline__ void rank_sort(const int *key_of, const int *val, OUT *out, int nl, int t0, int lane) {
 	int key[NQ], rnk[NQ];
 #pragma unroll
 	for (int q = 0; q < NQ; q++) {
@@ -303,7 +320,8 @@ __device__ __forceinline__ void rank_sort(const int *key_of, const int *val, int
 		key[q] = t < nl ? key_of[t] : 0x7fffffff;
 		rnk[q] = 0;
 	}
-#pragma unroll 4
+	constexpr int U = NQ > 4 ? 4 : 2;
+#pragma unroll U
 	for (int u = 0; u < nl; u++) {
 		const int x = key_of[u];
 #pragma unroll
@@ -314,6 +332,69 @@ __device__ __forceinline__ void rank_sort(const int *key_of, const int *val, int
 		const int t = t0 + q * 32 + lane;
 		if (t < nl) out[rnk[q]] = val[t];
 	}
+}
+
+// srt: the slots of the row's off-diagonal columns by ascending column.  A row
+// calls this before it waits for a member (the sort is off the critical chain
+// then) and once more before its finish; `sorted` of the columns were in order
+// by the last call, and as long as few came since they are merged in.
+template <int NQ, class WS>
+__device__ __forceinline__ void merge_columns(WS &s, int sorted, int d, int lane) {
+	int h[NQ], key[NQ], sh[NQ];
+#pragma unroll
+	for (int q = 0; q < NQ; q++) {
+		const int t = q * 32 + lane;
+		h[q] = t < sorted ? s.srt[t] : 0;
+		key[q] = t < sorted ? s.hkey[h[q]] : 0x7fffffff;
+		sh[q] = 0;
+	}
+	const int hn = lane < d ? s.slots[1 + sorted + lane] : 0;
+	const int kn = lane < d ? s.hkey[hn] : 0x7fffffff;
+	int at = 0;
+#pragma unroll 2
+	for (int j = 0; j < d; j++) {
+		const int x = __shfl_sync(0xffffffffu, kn, j);
+		int below = 0;
+#pragma unroll
+		for (int q = 0; q < NQ; q++) {
+			below += __popc(__ballot_sync(0xffffffffu, key[q] < x));
+			sh[q] += x < key[q];
+		}
+		at += x < kn;
+		if (lane == j) at += below;
+	}
+	__syncwarp();
+#pragma unroll
+	for (int q = 0; q < NQ; q++)
+		if (q * 32 + lane < sorted) s.srt[q * 32 + lane + sh[q]] = h[q];
+	if (lane < d) s.srt[at] = hn;
+	__syncwarp();
+}
+template <class WS>
+__device__ void sort_all(WS &s, int nc, int lane) {
+#pragma unroll 1
+	for (int t = lane; t < nc; t += 32) {
+		const int h = s.slots[1 + t];
+		s.lst[t] = h;
+		s.lkey[t] = s.hkey[h];
+	}
+	__syncwarp();
+	// each lane ranks its keys against one broadcast key per step
+	constexpr int NQ = WS::big ? 8 : 4;
+#pragma unroll 1
+	for (int t0 = 0; t0 < nc; t0 += 32 * NQ) rank_sort<NQ>(s.lkey, s.lst, s.srt, nc, t0, lane);
+	__syncwarp();
+}
+template <class WS>
+__device__ __forceinline__ void sort_columns(WS &s, int ncol, int &sorted, int lane) {
+	const int nc = ncol - 1, d = nc - sorted;
+	if (d == 0) return;
+	if (d <= 32 && sorted > 0 && sorted <= 128) {
+		merge_columns<4>(s, sorted, d, lane);
+	} else {
+		sort_all(s, nc, lane);
+	}
+	sorted = nc;
 }
 
 // Add a nonnegative compensation to row j's 64-bit fixed-point accumulator
@@ -342,6 +423,7 @@ __device__ void q_push(const FactArgs &A, int row) {
 	const unsigned long long t = atomicAdd(A.qtail, 1ull);
 	int *slot = A.queue + (t & (unsigned long long)(A.qcap - 1));
 	const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
 	for (unsigned it = 0; atomicCAS(slot, -1, row) != -1; it++) {
 		__nanosleep(64);
 		if ((it & 31) == 31 && globaltimer_ns() - t0 > BSG_SPIN_LIMIT_NS) {
@@ -361,6 +443,7 @@ __device__ int q_pop(const FactArgs &A) {
 	// warps still finish rows (a long chain of dependent rows) is progress
 	unsigned long long t0 = globaltimer_ns();
 	int seen = *(volatile int *)A.done_count;
+#pragma unroll 1
 	for (unsigned it = 1;; it++) {
 		__nanosleep(64);
 		if (*(volatile int *)slot >= 0) {
@@ -382,14 +465,25 @@ __device__ int q_pop(const FactArgs &A) {
 	}
 }
 
+// Rows queued and not yet taken by a warp (negative: warps wait for rows).
+__device__ __forceinline__ long long q_backlog(const FactArgs &A) {
+	return (long long)(*(volatile unsigned long long *)A.qtail - *(volatile unsigned long long *)A.qhead);
+}
+
 // Admission.  nstat[j] packs the static contributors of row j (the rows k
 // < j with A(k,j) != 0) that are unfinished (bits 0..14) and unclaimed (bits
 // 15..29); bit 30 marks j queued once, bit 31 claimed once.  Row j enters the
 // queue when all of them are claimed and at most one is unfinished: it then
-// starts while its last predecessor is being computed and waits for it.  A
-// row that another row waits for is queued earlier (promoted) if nobody has
-// queued it yet.  Bit 30 makes the first of the two the only one: a row is
-// queued once this way, and again only when a row it parked on finishes.
+// starts while its last predecessor is being computed and waits for it.  With
+// more than a sixteenth of the warps idle it enters with two unfinished: a row
+// takes tens of microseconds before its first wait, and one that starts late
+// holds up its chain; not while the global workspaces are in demand, where a
+// waiting row keeps one from the rows it waits for (IC2 32^3 18.2 -> 12.3 ms, 80x72x65 66.7 -> 54.4; always
+// with two unfinished, waiting rows take the warps that others need: 80x72x65
+// 206 ms, 128^3 1.3 s).  A row that another row waits for is queued earlier
+// (promoted) if nobody has queued it yet.  Bit 30 makes the first of these the
+// only one: a row is queued once this way, and again only when a row it parked
+// on finishes.
 #define ADM_ONE_FIN 1u
 #define ADM_ONE_CLAIM (1u << 15)
 #define ADM_QUEUED (1u << 30)
@@ -405,20 +499,31 @@ __device__ void enqueue_once(const FactArgs &A, int j) {
 }
 __device__ void admit_step(const FactArgs &A, int j, unsigned delta) {
 	const unsigned old = atomicSub(reinterpret_cast<unsigned *>(A.nstat) + j, delta);
-	if (!admissible(old) && admissible(old - delta)) enqueue_once(A, j);
+	const unsigned now = old - delta;
+	bool q = !admissible(old) && admissible(now);
+	if (delta == ADM_ONE_CLAIM && ((now >> 15) & 0x7fffu) == 0 && (now & 0x7fffu) == BSG_ADMIT_UNFINISHED + 1)
+		q = -q_backlog(A) > A.hold_max / 8 && *(volatile int *)A.nbig < BIG_SLOTS / 4;
+	if (q) enqueue_once(A, j);
 }
 
 // Wait (lane 0) for row m while a warp is computing it: 1 once m is
-// finished, 0 when nobody is computing m (the caller parks), -1 on the
-// spin limit or another warp's failure.
-__device__ int wait_row(const FactArgs &A, int m) {
+// finished (rec its record), 0 when nobody is computing m (the caller parks),
+// -1 on the spin limit or another warp's failure.  The record is polled alone,
+// one round trip to L2 a poll; the rest is looked at every eighth time.
+__device__ int wait_row(const FactArgs &A, int m, unsigned long long &rec) {
 	const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
 	for (unsigned it = 0;; it++) {
-		if (ld_acquire_u64(A.rec + m) & REC_DONE) return 1;
-		if (*(volatile int *)(A.inprog + m) == 0) return (ld_acquire_u64(A.rec + m) & REC_DONE) ? 1 : 0;
-		if (*(volatile int *)&A.st->code != 0) return -1;
+		rec = ld_acquire_u64(A.rec + m);
+		if (rec & REC_DONE) return 1;
 		__nanosleep(32);
-		if ((it & 63) == 63 && globaltimer_ns() - t0 > BSG_SPIN_LIMIT_NS) return -1;
+		if ((it & 7) != 7) continue;
+		if (*(volatile int *)(A.inprog + m) == 0) {
+			rec = ld_acquire_u64(A.rec + m);
+			return (rec & REC_DONE) ? 1 : 0;
+		}
+		if (*(volatile int *)&A.st->code != 0) return -1;
+		if (globaltimer_ns() - t0 > BSG_SPIN_LIMIT_NS) return -1;
 	}
 }
 
@@ -436,11 +541,6 @@ __device__ int promote(const FactArgs &A, int m) {
 		if (*(volatile int *)&A.st->code != 0 || globaltimer_ns() - t0 > PROMOTE_WAIT_NS) return 0;
 		__nanosleep(64);
 	}
-}
-
-// Rows queued and not yet taken by a warp (negative: warps wait for rows).
-__device__ __forceinline__ long long q_backlog(const FactArgs &A) {
-	return (long long)(*(volatile unsigned long long *)A.qtail - *(volatile unsigned long long *)A.qhead);
 }
 
 // Hold row i (lane 0) for member m that no warp computes right now (m is
@@ -465,6 +565,7 @@ __device__ int hold_for(const FactArgs &A, int m) {
 	}
 	const unsigned long long t0 = globaltimer_ns();
 	int res = 0;
+#pragma unroll 1
 	for (unsigned it = 0;; it++) {
 		if (ld_acquire_u64(A.rec + m) & REC_DONE) { res = 1; break; }
 		if ((it & 15) == 15) {
@@ -505,6 +606,7 @@ __device__ int close_pass(const FactArgs &A, WS &s, int i, int lane, int &levmax
 	int pm = 0x7fffffff;
 	int nd = 0;
 	// finished unclosed members: W index, pool offset, length (scratch in Ws/Wps/Wes)
+#pragma unroll 1
 	for (int base = 0; base < nW; base += 32) {
 		const int t = base + lane;
 		int m = -1;
@@ -530,6 +632,7 @@ __device__ int close_pass(const FactArgs &A, WS &s, int i, int lane, int &levmax
 	__syncwarp();
 	// chunk bases of the flattened rows
 	int T = 0;
+#pragma unroll 1
 	for (int d0 = 0; d0 < nd; d0 += 32) {
 		const int d = d0 + lane;
 		int tot;
@@ -544,19 +647,28 @@ __device__ int close_pass(const FactArgs &A, WS &s, int i, int lane, int &levmax
 	constexpr int NREG = 4;
 	uint4 reg[NREG];
 	int rown[NREG];
+	auto chunk = [&](int lo, int k) {
+		return __ldcg(reinterpret_cast<const uint4 *>(A.pool_cf + s.Wps[lo]) + (k - s.Wb[lo]));
+	};
+	// chunk k of round r (from the registers while they hold it)
+	auto pick = [&](int r, int k, int &lo, uint4 &v) {
+		if (r < NREG) {
+			lo = rown[0];
+			v = reg[0];
 #pragma unroll
-	for (int r = 0; r < NREG; r++) {
-		reg[r] = make_uint4(0u, 0u, 0u, 0u);
-		rown[r] = 0;
-	}
-	for (int k0 = 0, r = 0; k0 < T; k0 += 32, r++) {
-		const int k = k0 + lane;
-		if (k >= T) continue;
-		const int lo = seg_owner(s.Wb, nd, k);
-		const int ch = k - s.Wb[lo], len = s.Wes[lo];
-		const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(A.pool_cf + s.Wps[lo]) + ch);
+			for (int q = 1; q < NREG; q++)
+				if (q == r) {
+					v = reg[q];
+					lo = rown[q];
+				}
+		} else {
+			lo = seg_owner(s.Wb, nd, k);
+			v = chunk(lo, k);
+		}
+	};
+	auto find = [&](int lo, int k, const uint4 &v) { // column i and the depth in a chunk
+		const int ch = k - s.Wb[lo], len = s.Wes[lo], t = s.Ws[lo];
 		const unsigned e4[4] = {v.x, v.y, v.z, v.w};
-		const int t = s.Ws[lo];
 		if (ch == 0) s.Wlv[t] = CF_COL(e4[0]);
 #pragma unroll
 		for (int c = 0; c < 4; c++) {
@@ -566,53 +678,73 @@ __device__ int close_pass(const FactArgs &A, WS &s, int i, int lane, int &levmax
 				s.Wf[t] = (unsigned char)CF_FLAG(e4[c]);
 			}
 		}
+	};
 #pragma unroll
-		for (int q = 0; q < NREG; q++)
-			if (q == r) {
-				reg[q] = v;
-				rown[q] = lo;
-			}
+	for (int r = 0; r < NREG; r++) {
+		const int k = r * 32 + lane;
+		reg[r] = make_uint4(0u, 0u, 0u, 0u);
+		rown[r] = 0;
+		if (k < T) {
+			rown[r] = seg_owner(s.Wb, nd, k);
+			reg[r] = chunk(rown[r], k);
+		}
+	}
+#pragma unroll 1
+	for (int k0 = 0, r = 0; k0 < T; k0 += 32, r++) {
+		const int k = k0 + lane;
+		if (k >= T) continue;
+		int lo;
+		uint4 v;
+		pick(r, k, lo, v);
+		find(lo, k, v);
 	}
 	__syncwarp();
 	// the stored columns between the member and i become members
+#pragma unroll 1
 	for (int k0 = 0, r = 0; k0 < T && !err; k0 += 32, r++) {
 		const int k = k0 + lane;
 		unsigned e4[4] = {0u, 0u, 0u, 0u};
 		int pos = 0, ch = 0;
 		unsigned fi = F_D;
 		if (k < T) {
-			int lo = 0;
-			uint4 v = make_uint4(0u, 0u, 0u, 0u);
-			if (r < NREG) {
-#pragma unroll
-				for (int q = 0; q < NREG; q++)
-					if (q == r) {
-						v = reg[q];
-						lo = rown[q];
-					}
-			} else {
-				lo = seg_owner(s.Wb, nd, k);
-			}
+			int lo;
+			uint4 v;
+			pick(r, k, lo, v);
 			ch = k - s.Wb[lo];
 			const int t = s.Ws[lo];
 			fi = s.Wf[t];
 			if (fi != F_D) {
 				pos = s.Wp[t] - s.Wps[lo];
 				if (4 * ch < pos) {
-					if (r >= NREG) v = __ldcg(reinterpret_cast<const uint4 *>(A.pool_cf + s.Wps[lo]) + ch);
 					e4[0] = v.x; e4[1] = v.y; e4[2] = v.z; e4[3] = v.w;
 				}
 			}
 		}
-		unsigned fresh = 0; // bit c: entry c is a new member
+		// bit c of fresh: entry c is a new member.  The near rows' bits are
+		// looked at together, the far rows (rare) go one by one
+		unsigned fresh = 0, far = 0, clear = 0;
 #pragma unroll
 		for (int c = 0; c < 4; c++) {
-			const int e = 4 * ch + c;
+			const int e = 4 * ch + c, d = i - 1 - CF_COL(e4[c]);
 			if (e >= 1 && e < pos && !(fi == F_R && CF_FLAG(e4[c]) == F_R)) {
-				const int isnew = wset_insert(s, i, CF_COL(e4[c]));
-				if (isnew < 0) err = BSG_ERR_WORKSPACE;
-				else if (isnew) fresh |= 1u << c;
+				if (d >= WS::mwin) far |= 1u << c;
+				else if (!(s.wbits[d >> 5] & (1u << (d & 31)))) clear |= 1u << c;
 			}
+		}
+		if (clear) {
+#pragma unroll
+			for (int c = 0; c < 4; c++) {
+				const int d = i - 1 - CF_COL(e4[c]);
+				if ((clear & (1u << c)) && !(atomicOr(&s.wbits[d >> 5], 1u << (d & 31)) & (1u << (d & 31)))) fresh |= 1u << c;
+			}
+		}
+#pragma unroll 1
+		while (far) {
+			const int c = __ffs(far) - 1;
+			far &= far - 1;
+			const int isnew = wset_far(s, CF_COL(c < 2 ? (c ? e4[1] : e4[0]) : (c == 2 ? e4[2] : e4[3])));
+			if (isnew < 0) err = BSG_ERR_WORKSPACE;
+			else if (isnew) fresh |= 1u << c;
 		}
 		int tot;
 		const int ex = warp_excl_scan(__popc(fresh), lane, tot);
@@ -630,6 +762,7 @@ __device__ int close_pass(const FactArgs &A, WS &s, int i, int lane, int &levmax
 		err = __reduce_min_sync(0xffffffffu, err);
 	}
 	// closed: pool end, state, forward-solve depth through U members
+#pragma unroll 1
 	for (int d = lane; d < nd; d += 32) {
 		const int t = s.Ws[d];
 		s.We[t] = s.Wps[d] + s.Wes[d];
@@ -640,29 +773,67 @@ __device__ int close_pass(const FactArgs &A, WS &s, int i, int lane, int &levmax
 	return nd;
 }
 
+// The nb members listed in lsts, by row index, into Ws / Wps / Wes / Wfs; marked
+// applied.
+template <class WS>
+__device__ __forceinline__ void sort_members(WS &s, int nb, int lane) {
+	constexpr int NQ = WS::big ? 8 : 4;
+#pragma unroll 1
+	for (int q = lane; q < nb; q += 32) s.lkey[q] = s.W[s.lsts[q]];
+	__syncwarp();
+#pragma unroll 1
+	for (int t0 = 0; t0 < nb; t0 += 32 * NQ) rank_sort<NQ>(s.lkey, s.lsts, s.lst, nb, t0, lane);
+	__syncwarp();
+#pragma unroll 1
+	for (int r = lane; r < nb; r += 32) {
+		const int t = s.lst[r];
+		s.Ws[r] = s.W[t]; s.Wps[r] = s.Wp[t]; s.Wes[r] = s.We[t]; s.Wfs[r] = s.Wf[t];
+		s.Wst[t] = 2;
+	}
+}
+
+// The smallest member that is not closed (none: 0x7fffffff) and its place t, and
+// whether a smaller one is closed and not applied (the whole warp).
+template <class WS>
+__device__ __forceinline__ int smallest_open(WS &s, int lane, int &t, bool &pending) {
+	const int nW = min(s.sc[0], s.cmax);
+	int m = 0x7fffffff, at = 0, p = 0x7fffffff;
+#pragma unroll 1
+	for (int q = lane; q < nW; q += 32) {
+		const int k = s.W[q], st = s.Wst[q];
+		if (st == 0 && k < m) {
+			m = k;
+			at = q;
+		}
+		if (st == 1) p = min(p, k);
+	}
+	const int best = __reduce_min_sync(0xffffffffu, m);
+	t = __shfl_sync(0xffffffffu, at, __ffs(__ballot_sync(0xffffffffu, m == best)) - 1);
+	pending = __reduce_min_sync(0xffffffffu, p) < best;
+	return best;
+}
+
 // Apply the updates of the closed members below `bound` (all members below
 // it are known by then) in ascending order, in groups of consecutive members
 // whose segments fit the prefetch buffer; marks them applied.  Returns 0, or
 // a BSG_ERR_* code (uniform over the warp).
 template <class WS>
-__device__ int apply_members(const FactArgs &A, WS &s, int bound, int lane, PhaseClock &pc) {
+__device__ int apply_members(const FactArgs &A, WS &s, int bound, int lane, PhaseClock &pc, int &npend, int &ncol) {
 	constexpr bool ilu = WS::ilu;
 	const int nW = min(s.sc[0], s.cmax);
 	// compact the selected members (closed, below the bound) in index order
-	if (lane == 0) s.sc[2] = 0;
-	__syncwarp();
+	int nb = 0;
+#pragma unroll 1
 	for (int base = 0; base < nW; base += 32) {
 		const int t = base + lane;
 		const bool sel = t < nW && s.Wst[t] == 1 && s.W[t] < bound;
 		const unsigned b = __ballot_sync(0xffffffffu, sel);
-		const int pos0 = s.sc[2];
-		if (sel) s.lsts[pos0 + __popc(b & ((1u << lane) - 1))] = t;
-		__syncwarp();
-		if (lane == 0) s.sc[2] = pos0 + __popc(b);
-		__syncwarp();
+		if (sel) s.lsts[nb + __popc(b & ((1u << lane) - 1))] = t;
+		nb += __popc(b);
 	}
-	const int nb = s.sc[2];
+	__syncwarp();
 	if (nb == 0) return 0;
+	npend -= nb;
 	pc.v[FS_BATCHES]++;
 	pc.v[FS_CLOSED] += nb;
 	// rank sort by row index (rows are distinct); mark applied.  Up to 32
@@ -671,24 +842,20 @@ __device__ int apply_members(const FactArgs &A, WS &s, int bound, int lane, Phas
 		const int t = lane < nb ? s.lsts[lane] : 0;
 		const int k = lane < nb ? s.W[t] : 0x7fffffff;
 		int r = 0;
+#pragma unroll 4
 		for (int u = 0; u < nb; u++) r += __shfl_sync(0xffffffffu, k, u) < k;
 		if (lane < nb) {
 			s.Ws[r] = k; s.Wps[r] = s.Wp[t]; s.Wes[r] = s.We[t]; s.Wfs[r] = s.Wf[t];
 			s.Wst[t] = 2;
 		}
 	} else {
-		for (int q = lane; q < nb; q += 32) {
-			const int t = s.lsts[q], k = s.W[t];
-			int r = 0;
-			for (int u = 0; u < nb; u++) r += s.W[s.lsts[u]] < k;
-			s.Ws[r] = k; s.Wps[r] = s.Wp[t]; s.Wes[r] = s.We[t]; s.Wfs[r] = s.Wf[t];
-			s.Wst[t] = 2;
-		}
+		sort_members(s, nb, lane);
 	}
 	__syncwarp();
 	// segment bases: stored member t contributes its entries [pos, end)
 	{
 		int run = 0;
+#pragma unroll 1
 		for (int t0 = 0; t0 < nb; t0 += 32) {
 			const int t = t0 + lane;
 			int tot;
@@ -700,6 +867,7 @@ __device__ int apply_members(const FactArgs &A, WS &s, int bound, int lane, Phas
 		__syncwarp();
 	}
 	int err = 0;
+#pragma unroll 1
 	for (int t0 = 0; t0 < nb && !err;) {
 		int t1 = t0;
 		while (t1 < nb && s.Wb[t1 + 1] - s.Wb[t0] <= s.pfcap) t1++;
@@ -707,6 +875,7 @@ __device__ int apply_members(const FactArgs &A, WS &s, int bound, int lane, Phas
 		const int gb = s.Wb[t0], npf = s.Wb[t1] - gb;
 		long long g0 = clock64();
 		// prefetch: 4 independent loads per lane in flight
+#pragma unroll 1
 		for (int f0 = 0; f0 < npf; f0 += 128) {
 			unsigned c4[4];
 			double l4[4], u4[4];
@@ -737,26 +906,34 @@ __device__ int apply_members(const FactArgs &A, WS &s, int bound, int lane, Phas
 		long long g1 = clock64();
 		pc.v[FS_CYC_PF] += g1 - g0;
 		// phase A: accumulator slot of every entry, in parallel (R x R gets none)
-		for (int f = lane; f < npf; f += 32) {
-			const int lo = t0 + seg_owner(s.Wb + t0, t1 - t0, gb + f);
-			const unsigned cf = s.pf_cf[f];
+#pragma unroll 1
+		for (int f0 = 0; f0 < npf; f0 += 32) { // whole warp in every round (note_slots)
+			const int f = f0 + lane;
+			bool fresh = false;
 			short sl = -1;
-			if (!(s.Wfs[lo] == F_R && CF_FLAG(cf) == F_R)) {
-				int h = hfind_insert(s, CF_COL(cf));
-				if (h < 0) err = BSG_ERR_WORKSPACE; else sl = (short)h;
+			if (f < npf) {
+				const int lo = t0 + seg_owner(s.Wb + t0, t1 - t0, gb + f);
+				const unsigned cf = s.pf_cf[f];
+				if (!(s.Wfs[lo] == F_R && CF_FLAG(cf) == F_R)) {
+					const int h = hfind_insert(s, CF_COL(cf), fresh);
+					if (h < 0) err = BSG_ERR_WORKSPACE; else sl = (short)h;
+				}
+				s.pf_slot[f] = sl;
 			}
-			s.pf_slot[f] = sl;
+			note_slots(s, ncol, fresh, sl, lane);
 		}
 		err = __reduce_min_sync(0xffffffffu, err);
 		__syncwarp();
 		long long g2 = clock64();
 		pc.v[FS_CYC_PA] += g2 - g1;
 		// phase B: ascending members, fma(-l, g, f) per column
+#pragma unroll 1
 		for (int t = t0; t < t1 && !err; t++) {
 			if (s.Wfs[t] == F_D) continue;
 			const int b = s.Wb[t] - gb, seg = s.Wb[t + 1] - s.Wb[t];
 			const double lel = s.pf_l[b];
 			const double uel = ilu ? s.pf_u[b] : lel;
+#pragma unroll 1
 			for (int e = lane; e < seg; e += 32) {
 				const int sl = s.pf_slot[b + e];
 				if (sl < 0) continue;
@@ -777,9 +954,102 @@ __device__ int apply_members(const FactArgs &A, WS &s, int bound, int lane, Phas
 }
 
 
+// Close and apply the one member m that row i waited for (record rec, place tw
+// in the member set): every smaller member has been applied, so its update is
+// the next in order.  One load brings its columns and values (a lane an entry,
+// two for rows over 32 entries), where the general passes take two round trips
+// to L2 after reading the record again.  False: the row is longer than 64
+// entries, nothing done (the general passes take it).
+template <class WS>
+__device__ bool take_member(const FactArgs &A, WS &s, int i, int tw, unsigned long long rec, int lane, int &levmax,
+                            int &nopen, int &ncol, int &err) {
+	constexpr bool ilu = WS::ilu;
+	const int len = REC_LEN(rec);
+	const long long off = REC_OFF(rec);
+	if (len > 64) return false;
+	unsigned cf[2];
+	double l[2], u[2];
+#pragma unroll
+	for (int q = 0; q < 2; q++) {
+		const int e = q * 32 + lane;
+		cf[q] = 0;
+		l[q] = u[q] = 0.0;
+		if (e < len) {
+			cf[q] = __ldcg(A.pool_cf + off + e);
+			l[q] = __ldcg(A.pool_l + off + e);
+			if (ilu) u[q] = __ldcg(A.pool_u + off + e);
+		}
+	}
+	int pos = -1; // column i in the member's row
+	double lel = 0.0, uel = 0.0;
+	unsigned fi = F_D;
+#pragma unroll
+	for (int q = 0; q < 2; q++) {
+		const int e = q * 32 + lane;
+		const unsigned b = __ballot_sync(0xffffffffu, e >= 1 && e < len && CF_COL(cf[q]) == i);
+		if (b) {
+			const int at = __ffs(b) - 1;
+			pos = q * 32 + at;
+			fi = CF_FLAG(__shfl_sync(0xffffffffu, cf[q], at));
+			lel = __shfl_sync(0xffffffffu, l[q], at);
+			uel = ilu ? __shfl_sync(0xffffffffu, u[q], at) : lel;
+		}
+	}
+	if (lane == 0) s.Wst[tw] = 2;
+	nopen--;
+	if (pos >= 0) {
+		const int depth = CF_COL(__shfl_sync(0xffffffffu, cf[0], 0)); // entry 0 carries it
+		if (fi == F_U) levmax = max(levmax, depth + 1);
+#pragma unroll 1
+		for (int q = 0; q < 2 && 32 * q < len; q++) {
+			const int e = q * 32 + lane;
+			const unsigned cq = q ? cf[1] : cf[0];
+			const double lq = q ? l[1] : l[0], uq = q ? u[1] : u[0];
+			const bool use = e >= 1 && e < len && !(fi == F_R && CF_FLAG(cq) == F_R);
+			bool fresh = false, fcol = false;
+			int h = -1;
+			if (use && e < pos) {
+				const int isnew = wset_insert(s, i, CF_COL(cq));
+				if (isnew < 0) err = BSG_ERR_WORKSPACE;
+				fresh = isnew > 0;
+			} else if (use) {
+				h = hfind_insert(s, CF_COL(cq), fcol);
+				if (h < 0) err = BSG_ERR_WORKSPACE;
+				else if (ilu) {
+					s.hl[h] = fma(-uel, lq, s.hl[h]);
+					s.hu[h] = fma(-lel, uq, s.hu[h]);
+				} else {
+					s.hl[h] = fma(-lel, lq, s.hl[h]);
+				}
+			}
+			note_slots(s, ncol, fcol, h, lane);
+			const unsigned b = __ballot_sync(0xffffffffu, fresh);
+			if (b) {
+				const int q0 = s.sc[0], slot = q0 + __popc(b & ((1u << lane) - 1));
+				if (fresh) {
+					if (slot < s.cmax) {
+						s.W[slot] = CF_COL(cq);
+						s.Wst[slot] = 0;
+					} else {
+						err = BSG_ERR_WORKSPACE;
+					}
+				}
+				__syncwarp();
+				if (lane == 0) s.sc[0] = q0 + __popc(b);
+				nopen += __popc(b);
+			}
+			__syncwarp();
+		}
+	}
+	err = __reduce_min_sync(0xffffffffu, err);
+	__syncwarp();
+	return true;
+}
+
 // After row i is published: release the rows of A's row i, wake the rows
 // parked on i, count.
 __device__ void after_publish(const FactArgs &A, int i, int lane) {
+#pragma unroll 1
 	for (int k = A.iu[i] + 1 + lane; k < A.iu[i + 1]; k += 32) admit_step(A, A.ju[k], ADM_ONE_FIN);
 	if (lane == 0) {
 		__threadfence();
@@ -809,10 +1079,11 @@ __device__ __forceinline__ double *bv_l(WS &s, int h) { return s.hl + 9 * (s.hca
 // The scaled block row of A (Ilu2 / Ich2 init: scll_i A_ij scll_j^T, the
 // diagonal block with its scaling done).
 template <class WS>
-__device__ int init_blk(const FactArgs &A, WS &s, int i, int lane) {
-	int err = 0;
+__device__ int init_blk(const FactArgs &A, WS &s, int i, int lane, int &ncol) {
+	int err = 0, h = -1;
+	bool fresh = false;
 	if (lane == 0) {
-		const int h = hfind_insert(s, i);
+		h = hfind_insert(s, i, fresh);
 		double *u = bv_u(s, h);
 #pragma unroll
 		for (int k = 0; k < 9; k++) u[k] = __ldg(A.diag0 + 9 * (size_t)i + k);
@@ -822,15 +1093,17 @@ __device__ int init_blk(const FactArgs &A, WS &s, int i, int lane) {
 			for (int k = 0; k < 9; k++) l[k] = u[k];
 		}
 	}
+	note_slots(s, ncol, fresh, h, lane); // the diagonal comes first
 	__syncwarp();
 	const double *sli = A.scll + 9 * (size_t)i, *sui = A.sclu + 9 * (size_t)i;
-	for (int k = A.iu[i] + 1 + lane; k < A.iu[i + 1]; k += 32) {
-		const int j = A.ju[k];
-		const int h = hfind_insert(s, j);
-		if (h < 0) {
-			err = BSG_ERR_WORKSPACE;
-			continue;
-		}
+#pragma unroll 1
+	for (int k0 = A.iu[i] + 1; k0 < A.iu[i + 1]; k0 += 32) {
+		const int k = k0 + lane, j = k < A.iu[i + 1] ? A.ju[k] : -1;
+		fresh = false;
+		h = j >= 0 ? hfind_insert(s, j, fresh) : -1;
+		if (j >= 0 && h < 0) err = BSG_ERR_WORKSPACE;
+		note_slots(s, ncol, fresh, h, lane);
+		if (h < 0) continue;
 		double t[9];
 		mm3(sli, 1, 3, A.au + 9 * (size_t)k, 1, 3, t);
 		mm3(t, 1, 3, A.sclu + 9 * (size_t)j, 3, 1, bv_u(s, h));
@@ -850,35 +1123,28 @@ __device__ int init_blk(const FactArgs &A, WS &s, int i, int lane) {
 // The lanes take the blocks of one member (distinct columns), the members
 // go in order, so the sums do not depend on the schedule.
 template <class WS>
-__device__ int apply_blk(const FactArgs &A, WS &s, int bound, int lane, PhaseClock &pc) {
+__device__ int apply_blk(const FactArgs &A, WS &s, int bound, int lane, PhaseClock &pc, int &npend, int &ncol) {
 	constexpr bool ilu = WS::ilu;
 	const int nW = min(s.sc[0], s.cmax);
-	if (lane == 0) s.sc[2] = 0;
-	__syncwarp();
+	int nb = 0;
+#pragma unroll 1
 	for (int base = 0; base < nW; base += 32) {
 		const int t = base + lane;
 		const bool sel = t < nW && s.Wst[t] == 1 && s.W[t] < bound;
 		const unsigned b = __ballot_sync(0xffffffffu, sel);
-		const int pos0 = s.sc[2];
-		if (sel) s.lsts[pos0 + __popc(b & ((1u << lane) - 1))] = t;
-		__syncwarp();
-		if (lane == 0) s.sc[2] = pos0 + __popc(b);
-		__syncwarp();
+		if (sel) s.lsts[nb + __popc(b & ((1u << lane) - 1))] = t;
+		nb += __popc(b);
 	}
-	const int nb = s.sc[2];
+	__syncwarp();
 	if (nb == 0) return 0;
+	npend -= nb;
 	pc.v[FS_BATCHES]++;
 	pc.v[FS_CLOSED] += nb;
-	for (int q = lane; q < nb; q += 32) {
-		const int t = s.lsts[q], k = s.W[t];
-		int r = 0;
-		for (int u = 0; u < nb; u++) r += s.W[s.lsts[u]] < k;
-		s.Ws[r] = k; s.Wps[r] = s.Wp[t]; s.Wes[r] = s.We[t]; s.Wfs[r] = s.Wf[t];
-		s.Wst[t] = 2;
-	}
+	sort_members(s, nb, lane);
 	__syncwarp();
 	const double *pg_l = A.pool_l, *pg_u = ilu ? A.pool_u : A.pool_l;
 	int err = 0;
+#pragma unroll 1
 	for (int t = 0; t < nb && !err; t++) {
 		if (s.Wfs[t] == F_D) continue;
 		const long long q = s.Wps[t], end = s.Wes[t];
@@ -889,20 +1155,24 @@ __device__ int apply_blk(const FactArgs &A, WS &s, int bound, int lane, PhaseClo
 			lel[k] = __ldcg(pg_l + 9 * q + k);
 			uel[k] = ilu ? __ldcg(pg_u + 9 * q + k) : 0.0;
 		}
-		for (long long e = q + lane; e < end; e += 32) {
-			const unsigned cf = __ldcg(A.pool_cf + e);
-			if (rr && CF_FLAG(cf) == F_R) continue;
+#pragma unroll 1
+		for (long long e0 = q; e0 < end; e0 += 32) {
+			const long long e = e0 + lane;
+			const unsigned cf = e < end ? __ldcg(A.pool_cf + e) : 0u;
+			const bool use = e < end && !(rr && CF_FLAG(cf) == F_R);
+			bool fresh = false;
 			double gu[9], gl[9];
+			if (use) {
 #pragma unroll
-			for (int k = 0; k < 9; k++) {
-				gu[k] = __ldcg(pg_u + 9 * e + k);
-				gl[k] = ilu ? __ldcg(pg_l + 9 * e + k) : 0.0;
+				for (int k = 0; k < 9; k++) {
+					gu[k] = __ldcg(pg_u + 9 * e + k);
+					gl[k] = ilu ? __ldcg(pg_l + 9 * e + k) : 0.0;
+				}
 			}
-			const int h = hfind_insert(s, CF_COL(cf));
-			if (h < 0) {
-				err = BSG_ERR_WORKSPACE;
-				continue;
-			}
+			const int h = use ? hfind_insert(s, CF_COL(cf), fresh) : -1;
+			if (use && h < 0) err = BSG_ERR_WORKSPACE;
+			note_slots(s, ncol, fresh, h, lane);
+			if (h < 0) continue;
 			double tu[9];
 			mm3(lel, 3, 1, gu, 1, 3, tu); // gl_q^T gu_e
 			double *u = bv_u(s, h);
@@ -932,25 +1202,25 @@ __device__ int apply_blk(const FactArgs &A, WS &s, int bound, int lane, PhaseClo
 // stored as U (max-norm >= tau1) or R in ascending column order.
 template <class WS>
 __device__ int finish_blk(const FactArgs &A, WS &s, int i, int lane, int levmax, unsigned long long accraw,
-                          PhaseClock &pc, long long tail0) {
+                          PhaseClock &pc, long long tail0, int ncol) {
 	constexpr bool ilu = WS::ilu;
 	// the three received compensations (lanes 0..2)
 	const double comp = __dmul_rn((double)accraw, A.acc_inv_scale);
-	// ---- filter, in slot order: blocks of max-norm below tau2 are dropped,
-	//      theta times their entries going to this row's pivot block (row
-	//      sums, added exactly in fixed point, so their order does not
+	// ---- filter, by ascending column: blocks of max-norm below tau2 are
+	//      dropped, theta times their entries going to this row's pivot block
+	//      (row sums, added exactly in fixed point, so their order does not
 	//      matter) and to the dropped column's pivot block; the kept ones
-	//      are listed in lsts / lkey
+	//      are listed in lsts.  A global workspace, with its thousands of
+	//      columns not in order, goes by insertion and sorts the kept ones
 	unsigned long long rq0 = 0, rq1 = 0, rq2 = 0;
-	int nl = 0;
-	if (lane == 0) s.sc[2] = 0;
-	__syncwarp();
-	const int hscan = WS::big ? s.sc[3] : s.hcap; // slots to look at
-	for (int q0 = 0; q0 < hscan; q0 += 32) { // whole warp in every round (ballots)
+	const int nl = ncol - 1;
+	int nk = 0;
+#pragma unroll 1
+	for (int q0 = 0; q0 < nl; q0 += 32) {
 		const int q = q0 + lane;
-		const int h = q < hscan ? (WS::big ? s.slots[q] : q) : -1;
-		const int c = h >= 0 ? s.hkey[h] : -1;
-		const bool take = c >= 0 && c != i;
+		const bool take = q < nl;
+		const int h = take ? (WS::big ? s.slots[1 + q] : s.srt[q]) : 0;
+		const int c = take ? s.hkey[h] : -1;
 		bool keep = false;
 		if (take) {
 			const double *u = bv_u(s, h), *l = ilu ? bv_l(s, h) : u;
@@ -977,16 +1247,18 @@ __device__ int finish_blk(const FactArgs &A, WS &s, int i, int lane, int levmax,
 				acc_push(A.acc, 3 * c + 2, cs2, A.acc_scale, A.st);
 			}
 		}
-		nl += __popc(__ballot_sync(0xffffffffu, take));
 		const unsigned b = __ballot_sync(0xffffffffu, keep);
-		const int base = s.sc[2];
 		if (keep) {
-			const int at = base + __popc(b & ((1u << lane) - 1));
+			const int at = nk + __popc(b & ((1u << lane) - 1));
 			s.lsts[at] = h;
-			s.lkey[at] = c;
+			if (WS::big) s.lkey[at] = c;
 		}
-		__syncwarp();
-		if (lane == 0) s.sc[2] = base + __popc(b);
+		nk += __popc(b);
+	}
+	__syncwarp();
+	if (WS::big) {
+#pragma unroll 1
+		for (int t0 = 0; t0 < nk; t0 += 256) rank_sort<8>(s.lkey, s.lsts, s.lst, nk, t0, lane);
 		__syncwarp();
 	}
 #pragma unroll
@@ -997,15 +1269,7 @@ __device__ int finish_blk(const FactArgs &A, WS &s, int i, int lane, int levmax,
 	}
 	const double rs0 = __dmul_rn((double)rq0, A.acc_inv_scale), rs1 = __dmul_rn((double)rq1, A.acc_inv_scale),
 	             rs2 = __dmul_rn((double)rq2, A.acc_inv_scale);
-	const int nk = s.sc[2];
-	// ---- the kept columns ascending (rank sort): lst
-	if (nk <= 32) rank_sort<1>(s.lkey, s.lsts, s.lst, nk, 0, lane);
-	else if (nk <= 64) rank_sort<2>(s.lkey, s.lsts, s.lst, nk, 0, lane);
-	else if (nk <= 128) rank_sort<4>(s.lkey, s.lsts, s.lst, nk, 0, lane);
-	else
-		for (int t0 = 0; t0 < nk; t0 += 256) rank_sort<8>(s.lkey, s.lsts, s.lst, nk, t0, lane);
-	__syncwarp();
-	const int di = hfind_insert(s, i);
+	const int di = s.slots[0]; // the diagonal
 	const double c0 = __shfl_sync(0xffffffffu, comp, 0), c1 = __shfl_sync(0xffffffffu, comp, 1),
 	             c2 = __shfl_sync(0xffffffffu, comp, 2);
 	const int len = nk + 1;
@@ -1062,8 +1326,9 @@ __device__ int finish_blk(const FactArgs &A, WS &s, int i, int lane, int levmax,
 		A.pool_l[9 * off + lane] = dl[c + 3 * r];
 		if (ilu) A.pool_u[9 * off + lane] = du[c + 3 * r];
 	}
+#pragma unroll 1
 	for (int t = lane; t < nk; t += 32) {
-		const int h = s.lst[t];
+		const int h = WS::big ? s.lst[t] : s.lsts[t];
 		const double *u = bv_u(s, h), *l = ilu ? bv_l(s, h) : u;
 		double tu[9], tl[9];
 		mm3(dl, 1, 3, u, 1, 3, tu);
@@ -1084,8 +1349,7 @@ __device__ int finish_blk(const FactArgs &A, WS &s, int i, int lane, int levmax,
 		}
 	}
 	if (lane == 0) A.lev[i] = levmax;
-	__threadfence();
-	__syncwarp();
+	__syncwarp(); // the release below covers the whole warp's stores
 	if (lane == 0) st_release_u64(A.rec + i, REC_DONE | ((unsigned long long)off << 32) | (unsigned long long)len);
 	__syncwarp();
 	const long long cpub = clock64();
@@ -1104,20 +1368,28 @@ __device__ int finish_blk(const FactArgs &A, WS &s, int i, int lane, int levmax,
 // Pipelined: the row closes the members that are finished, applies the
 // updates of every closed member below the smallest unfinished one (the
 // members below it are all known: a member is only discovered from a
-// smaller member), then waits for that member while a warp computes it.
-// When the last predecessor finishes, only its own segment and the finish
-// are left.
+// smaller member), then waits for that member while a warp computes it,
+// closes and applies it alone (take_member) and goes on to the next.  When the
+// last predecessor finishes, only its own update and the finish are left: about
+// 5 us from one row's record to the next one's in an unbroken chain, of which
+// two round trips to L2 (the record, then the row) and the release 1.5 us.
+//
+// Code size counts as much as instruction count here: under load the 12 warps
+// of an SM sit in different parts of the row, and code that runs once a row
+// came from L2 (the pivot's square root and division took 224 cycles alone and
+// 806 under load).  Hence the loops that are not unrolled and the single call
+// sites: 319 KB of kernel -> 141 KB took 128^3 from 230 to 165 ms.
 template <class WS>
 __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc) {
 	constexpr bool ilu = WS::ilu;
 	const long long c0 = clock64();
 	for (int t = lane; t < s.wcap; t += 32) s.wset[t] = -1;
-	if (lane == 0) s.sc[3] = 0;
 	for (int t = lane; t < WS::mwin / 32; t += 32) s.wbits[t] = 0u; // (no bitmap: mwin 0)
 	for (int t = lane; t < s.hcap; t += 32) s.hkey[t] = -1;
 	if (lane == 0) s.sc[0] = 0;
 	__syncwarp();
 
+	int ncol = 0; // columns in the accumulator, the diagonal first
 	// ---- seed with A's column i
 	const int tb = A.it[i], te = A.it[i + 1];
 	if (te - tb > s.cmax) {
@@ -1125,6 +1397,7 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 		if (lane == 0) devstat_fail(A.st, BSG_ERR_WORKSPACE, i, 2);
 		return -2;
 	}
+#pragma unroll 1
 	for (int t = tb + lane; t < te; t += 32) {
 		int k = A.jt[t];
 		s.W[t - tb] = k;
@@ -1139,25 +1412,34 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 	int err = 0;
 	const int ab = A.iu[i], ae = A.iu[i + 1];
 	if constexpr (WS::blk) {
-		err = init_blk(A, s, i, lane);
+		err = init_blk(A, s, i, lane, ncol);
 		if (err) {
 			if (!WS::big) return -3;
 			if (lane == 0) devstat_fail(A.st, err, i, 4);
 			return -2;
 		}
 	} else {
-	if (lane == 0) {
-		int slot = hfind_insert(s, i);
-		s.hl[slot] = A.diag0[i];
-		if (ilu) s.hu[slot] = A.diag0[i];
+	{
+		bool fresh = false;
+		int slot = -1;
+		if (lane == 0) {
+			slot = hfind_insert(s, i, fresh);
+			s.hl[slot] = A.diag0[i];
+			if (ilu) s.hu[slot] = A.diag0[i];
+		}
+		note_slots(s, ncol, fresh, slot, lane);
 	}
 	__syncwarp();
 	{
 		const double si_l = A.scll[i], si_u = A.sclu[i];
-		for (int k = ab + 1 + lane; k < ae; k += 32) {
-			int j = A.ju[k];
-			int sl = hfind_insert(s, j);
-			if (sl < 0) { err = BSG_ERR_WORKSPACE; continue; }
+#pragma unroll 1
+		for (int k0 = ab + 1; k0 < ae; k0 += 32) {
+			const int k = k0 + lane, j = k < ae ? A.ju[k] : -1;
+			bool fresh = false;
+			const int sl = j >= 0 ? hfind_insert(s, j, fresh) : -1;
+			if (j >= 0 && sl < 0) err = BSG_ERR_WORKSPACE;
+			note_slots(s, ncol, fresh, sl, lane);
+			if (sl < 0) continue;
 			if (ilu) {
 				s.hl[sl] = __dmul_rn(__dmul_rn(A.al[k], si_u), A.scll[j]);
 				s.hu[sl] = __dmul_rn(__dmul_rn(A.au[k], si_l), A.sclu[j]);
@@ -1178,27 +1460,38 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 	int levmax = 0;
 	unsigned long long accraw = 0;
 	bool waited = false;
+	int nopen = te - tb, npend = 0; // members not closed, members closed and not applied
+	int sorted = 0;                 // columns in order, see sort_columns
 	long long tail0 = clock64(); // end of the last wait: the row's own latency starts here
+	// members that are waited for are taken alone, but for block rows and the
+	// rows of the global workspaces, whose thousands of members come in passes
+	constexpr bool alone = !WS::blk && !WS::big;
+	bool pass = true; // close passes (else the members are looked through for the next one)
 	for (;;) {
 		// ---- close the finished members, pass after pass, until a pass
 		//      closes none; the smallest member left is the bound
 		// (a pass that closed members but discovered none leaves nothing
 		// for another pass: every member is known, and the ones it found
 		// unfinished are waited for below)
-		int bound = i;
+		int bound = i, tw = -1;
+		bool pending = npend > 0;
 		const long long k0 = clock64();
-		for (;;) {
+		while (pass && nopen > 0) {
 			pc.v[FS_ROUNDS]++;
 			int pmin = 0x7fffffff, added = 0;
 			const long long q0 = clock64();
 			const int closed = close_pass(A, s, i, lane, levmax, pmin, err, added);
+			nopen += added - closed;
+			npend += closed;
 			pc.v[FS_CYC_PCLOSE] += clock64() - q0;
+			pending = npend > 0;
 			if (err) break;
 			if (!closed || !added) {
 				bound = pmin == 0x7fffffff ? i : pmin;
 				break;
 			}
 		}
+		if (alone && nopen > 0) bound = smallest_open(s, lane, tw, pending);
 		if (err) {
 			if (!WS::big) return -3;
 			if (lane == 0) devstat_fail(A.st, err, i, 3);
@@ -1210,10 +1503,12 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 		// the compensations received so far (every member seen finished has
 		// pushed its own before publishing): loaded now, used after the last
 		// pass, so the load overlaps the updates
-		if (lane < (WS::blk ? 3 : 1)) accraw = __ldcg(A.acc + (WS::blk ? 3 * (size_t)i + lane : (size_t)i));
+		if (pass && lane < (WS::blk ? 3 : 1)) accraw = __ldcg(A.acc + (WS::blk ? 3 * (size_t)i + lane : (size_t)i));
 		// ---- updates of the closed members below the bound
-		if constexpr (WS::blk) err = apply_blk(A, s, bound, lane, pc);
-		else err = apply_members(A, s, bound, lane, pc);
+		if (pending) {
+			if constexpr (WS::blk) err = apply_blk(A, s, bound, lane, pc, npend, ncol);
+			else err = apply_members(A, s, bound, lane, pc, npend, ncol);
+		}
 		const long long k2 = clock64();
 		pc.v[FS_CYC_UPD] += k2 - k1;
 		if (err) {
@@ -1221,16 +1516,28 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 			if (lane == 0) devstat_fail(A.st, err, i, 5);
 			return -2;
 		}
-		if (bound == i) break;
 		// ---- wait for the smallest unfinished member while a warp computes
-		//      it; park when nobody does
-		int res = 0;
-		if (lane == 0) {
-			res = wait_row(A, bound);
-			if (res == 0 && promote(A, bound)) res = wait_row(A, bound);
-			if (res == 0) res = hold_for(A, bound);
+		//      it; park when nobody does.  What the finish needs in order is
+		//      put in order meanwhile
+		unsigned long long rec = 0;
+		if (bound != i) {
+			if (lane == 0) rec = ld_acquire_u64(A.rec + bound);
+			rec = __shfl_sync(0xffffffffu, rec, 0);
+		}
+		if (WS::big ? bound == i && !WS::blk : bound == i || !(rec & REC_DONE)) sort_columns(s, ncol, sorted, lane);
+		if (bound == i) break;
+		const bool seen = (rec & REC_DONE) != 0;
+		int res = 1;
+		if (lane == 0 && !(rec & REC_DONE)) {
+			res = wait_row(A, bound, rec);
+			if (res == 0 && promote(A, bound)) res = wait_row(A, bound, rec);
+			if (res == 0) {
+				res = hold_for(A, bound);
+				if (res == 1) rec = ld_acquire_u64(A.rec + bound);
+			}
 		}
 		res = __shfl_sync(0xffffffffu, res, 0);
+		rec = __shfl_sync(0xffffffffu, rec, 0);
 		tail0 = clock64();
 		waited = true;
 		pc.v[FS_CYC_BLOCKED] += tail0 - k2;
@@ -1239,96 +1546,74 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 			if (lane == 0) devstat_fail(A.st, BSG_ERR_TIMEOUT, i, 7);
 			return -2;
 		}
+		pass = true;
+		if constexpr (alone) {
+			if (lane == 0) accraw = __ldcg(A.acc + i); // complete if this was the last member
+			if (take_member(A, s, i, tw, rec, lane, levmax, nopen, ncol, err)) {
+				pc.v[FS_CLOSED]++;
+				// the next one alone again, unless this one needed no wait: then
+				// more of them may have finished
+				pass = seen && nopen >= 2;
+			}
+			if (err) {
+				if (!WS::big) return -3;
+				if (lane == 0) devstat_fail(A.st, err, i, 5);
+				return -2;
+			}
+		}
 	}
 	levmax = __reduce_max_sync(0xffffffffu, levmax);
 	pc.v[FS_CONTRIB] += min(s.sc[0], s.cmax);
-	if constexpr (WS::blk) return finish_blk(A, s, i, lane, levmax, accraw, pc, tail0);
+	if constexpr (WS::blk) return finish_blk(A, s, i, lane, levmax, accraw, pc, tail0, ncol);
+	const int di = s.slots[0]; // the diagonal
 	{
 		const double comp = __dmul_rn((double)__shfl_sync(0xffffffffu, accraw, 0), A.acc_inv_scale);
 		if (lane == 0) {
-			const int di0 = hfind_insert(s, i);
-			s.hl[di0] = __dadd_rn(s.hl[di0], comp);
-			if (ilu) s.hu[di0] = __dadd_rn(s.hu[di0], comp);
+			s.hl[di] = __dadd_rn(s.hl[di], comp);
+			if (ilu) s.hu[di] = __dadd_rn(s.hu[di], comp);
 		}
-		__syncwarp();
 	}
 	const long long c3 = clock64();
 	(void)c0;
+	const int nl = sorted; // the off-diagonal columns, all in order now
 
-	// ---- extract the off-diagonal mask columns and sort them ascending
-	if (lane == 0) s.sc[1] = 0;
-	__syncwarp();
-	const int hscan = WS::big ? s.sc[3] : s.hcap; // slots to look at
-	for (int q0 = 0; q0 < hscan; q0 += 32) { // whole warp in every round (ballots)
-		const int q = q0 + lane;
-		const int h = q < hscan ? (WS::big ? s.slots[q] : q) : -1;
-		int c = h >= 0 ? s.hkey[h] : -1;
-		bool take = c >= 0 && c != i;
-		unsigned b = __ballot_sync(0xffffffffu, take);
-		int base = s.sc[1];
-		if (take) {
-			const int at = base + __popc(b & ((1u << lane) - 1));
-			s.lst[at] = h;
-			s.lkey[at] = c;
-		}
-		__syncwarp();
-		if (lane == 0) s.sc[1] = base + __popc(b);
-		__syncwarp();
-	}
-	const int nl = s.sc[1];
-	// rank sort (columns are distinct): each lane ranks its keys (as few per
-	// lane as the row needs) against one broadcast key per step
-	if (nl <= 32) rank_sort<1>(s.lkey, s.lst, s.lsts, nl, 0, lane);
-	else if (nl <= 64) rank_sort<2>(s.lkey, s.lst, s.lsts, nl, 0, lane);
-	else if (nl <= 128) rank_sort<4>(s.lkey, s.lst, s.lsts, nl, 0, lane);
-	else
-		for (int t0 = 0; t0 < nl; t0 += 256) rank_sort<8>(s.lkey, s.lst, s.lsts, nl, t0, lane);
-	__syncwarp();
-	const int di = hfind_insert(s, i); // existing slot of the diagonal
-
-	// ---- filter by tau2 with theta compensation (ascending columns): the
-	//      compensations of the dropped columns are formed in parallel (in
-	//      pf_l), the kept columns compacted into lst[] in ascending order,
-	//      and lane 0 adds the compensations to the diagonal in column order
-	if (lane == 0) s.sc[2] = 0;
-	__syncwarp();
+	// ---- filter by tau2 with theta compensation (ascending columns): the kept
+	//      slots are compacted into lst[] and the compensations of the dropped
+	//      ones into pf_l[], both in column order, and each compensation goes to
+	//      its column's row (the reductions are done by the time this row
+	//      publishes, and rows read a row's pushes only after acquiring its
+	//      record)
+	int nk = 0, nd = 0;
+#pragma unroll 1
 	for (int t0 = 0; t0 < nl; t0 += 32) {
 		const int t = t0 + lane;
-		bool keep = false;
-		if (t < nl) {
-			const int h = s.lsts[t];
-			double v = fabs(s.hl[h]);
-			if (ilu) v = fmax(v, fabs(s.hu[h]));
-			keep = v >= A.tau2;
-			s.pf_l[t] = keep ? 0.0 : __dmul_rn(v, A.theta);
+		const int h = t < nl ? s.srt[t] : 0;
+		double v = fabs(s.hl[h]);
+		if (ilu) v = fmax(v, fabs(s.hu[h]));
+		const bool keep = t < nl && v >= A.tau2, drop = t < nl && !keep;
+		const unsigned bk = __ballot_sync(0xffffffffu, keep), bd = __ballot_sync(0xffffffffu, drop);
+		if (keep) s.lst[nk + __popc(bk & ((1u << lane) - 1))] = h;
+		if (drop) {
+			const double w = __dmul_rn(v, A.theta);
+			s.pf_l[nd + __popc(bd & ((1u << lane) - 1))] = w;
+			if (w != 0.0) acc_push(A.acc, s.hkey[h], w, A.acc_scale, A.st);
 		}
-		const unsigned b = __ballot_sync(0xffffffffu, keep);
-		const int base = s.sc[2];
-		if (keep) s.lst[base + __popc(b & ((1u << lane) - 1))] = s.lsts[t];
-		__syncwarp();
-		if (lane == 0) s.sc[2] = base + __popc(b);
-		__syncwarp();
+		nk += __popc(bk);
+		nd += __popc(bd);
 	}
+	if (lane < (-nd & 7)) s.pf_l[nd + lane] = 0.0; // whole groups of 8 below
 	// the stored length is known: reserve the pool space now, so the
 	// atomic's round trip overlaps the compensation sum and the pivot
-	const int len = s.sc[2] + 1;
+	const int len = nk + 1;
 	const int alloc = (len + 3) & ~3;
 	long long off = 0;
 	if (lane == 0) off = (long long)atomicAdd(A.pool_len, (unsigned long long)alloc);
-	// ---- hand the dropped entries' compensations to their rows now: the
-	//      reductions are done by the time this row publishes (rows read a
-	//      row's pushes only after acquiring its record)
-	for (int t = lane; t < nl; t += 32) {
-		const double v = s.pf_l[t];
-		if (v != 0.0) acc_push(A.acc, s.hkey[s.lsts[t]], v, A.acc_scale, A.st);
-	}
-	// ---- the row's own compensations into its diagonal, in ascending column
-	//      order; a kept column contributes +0.0, which leaves the (positive)
-	//      sum unchanged, so the adds need no branch and the loads run ahead
+	__syncwarp();
+	// ---- the row's own compensations into its diagonal, in ascending column order
 	if (lane == 0) {
 		double dl = s.hl[di], du = ilu ? s.hu[di] : 0.0;
-		int t = 0;
-		for (; t + 8 <= nl; t += 8) {
+#pragma unroll 1
+		for (int t = 0; t < nd; t += 8) {
 			double v[8];
 #pragma unroll
 			for (int q = 0; q < 8; q++) v[q] = s.pf_l[t + q];
@@ -1338,16 +1623,10 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 				if (ilu) du = __dadd_rn(du, v[q]);
 			}
 		}
-		for (; t < nl; t++) {
-			const double v = s.pf_l[t];
-			dl = __dadd_rn(dl, v);
-			if (ilu) du = __dadd_rn(du, v);
-		}
 		s.hl[di] = dl;
 		if (ilu) s.hu[di] = du;
 	}
 	__syncwarp();
-	const int nk = s.sc[2];
 
 	// ---- pivot (Ich2PivScaleRow / Ilu2PivScaleRow)
 	const double fd = s.hl[di];
@@ -1377,6 +1656,7 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 		A.pool_l[off] = deleml;
 		if (ilu) A.pool_u[off] = delemu;
 	}
+#pragma unroll 1
 	for (int t = lane; t < nk; t += 32) {
 		const int h = s.lst[t];
 		double l = s.hl[h], u = ilu ? s.hu[h] : l;
@@ -1389,8 +1669,7 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 		if (ilu) A.pool_u[off + 1 + t] = u;
 	}
 	if (lane == 0) A.lev[i] = levmax;
-	__threadfence();
-	__syncwarp();
+	__syncwarp(); // the release below covers the whole warp's stores
 	if (lane == 0) st_release_u64(A.rec + i, REC_DONE | ((unsigned long long)off << 32) | (unsigned long long)len);
 	__syncwarp();
 	const long long cpub = clock64();
@@ -1434,6 +1713,7 @@ __global__ void __launch_bounds__((BLK ? FACT_WARPS_BLK : FACT_WARPS) * 32, FACT
 		if (lane == 0) first = !(atomicOr(reinterpret_cast<unsigned *>(A.nstat) + i, ADM_CLAIMED) & ADM_CLAIMED);
 		first = __shfl_sync(0xffffffffu, first, 0);
 		if (first)
+#pragma unroll 1
 			for (int k = A.iu[i] + 1 + lane; k < A.iu[i + 1]; k += 32) admit_step(A, A.ju[k], ADM_ONE_CLAIM);
 		__syncwarp();
 		int r = try_row(A, s, i, lane, pc);
@@ -1449,6 +1729,7 @@ __global__ void __launch_bounds__((BLK ? FACT_WARPS_BLK : FACT_WARPS) * 32, FACT
 					const int q = (start + k) % BIG_SLOTS;
 					if (atomicCAS(A.big_owner + q, 0, 1) == 0) slot = q;
 				}
+				if (slot >= 0) atomicAdd(A.nbig, 1);
 			}
 			slot = __shfl_sync(0xffffffffu, slot, 0);
 			if (slot < 0) {
@@ -1467,6 +1748,7 @@ __global__ void __launch_bounds__((BLK ? FACT_WARPS_BLK : FACT_WARPS) * 32, FACT
 			if (lane == 0) {
 				__threadfence();
 				atomicExch(A.big_owner + slot, 0);
+				atomicSub(A.nbig, 1);
 			}
 		}
 		if (r == -2) break;
@@ -1722,9 +2004,10 @@ int bsg_fact_run(bsg_ctx *c, bsg_mat *m, int kind, const bsg_param *p, bsg_fct *
 	if (grid < 1) grid = 1;
 	if (cudaMallocAsync(&A.big_ws, GlobWS<true>::bytes * (size_t)BIG_SLOTS, st) != cudaSuccess)
 		return bsg_set_error(BSG_ERR_NOMEM, "factor row workspace");
-	BSG_CUDA(cudaMallocAsync(&A.big_owner, sizeof(int) * (BIG_SLOTS + 1), st));
-	BSG_CUDA(cudaMemsetAsync(A.big_owner, 0, sizeof(int) * (BIG_SLOTS + 1), st));
+	BSG_CUDA(cudaMallocAsync(&A.big_owner, sizeof(int) * (BIG_SLOTS + 2), st));
+	BSG_CUDA(cudaMemsetAsync(A.big_owner, 0, sizeof(int) * (BIG_SLOTS + 2), st));
 	A.nhold = A.big_owner + BIG_SLOTS;
+	A.nbig = A.nhold + 1;
 	A.hold_max = grid * FACT_WARPS / 2;
 	kern<<<grid, FACT_WARPS * 32, smem, st>>>(A);
 	BSG_CUDA(cudaGetLastError());
@@ -1861,8 +2144,9 @@ int bsg_bfact_dyn(bsg_ctx *c, int nb, int sym, const bsg_param *p, const int *bi
 	A.qhead = qhead; A.qtail = qtail; A.done_count = done_count; A.st = c->d_stat;
 	if (cudaMallocAsync(&A.big_ws, big * (size_t)BIG_SLOTS, st) != cudaSuccess)
 		return bsg_set_error(BSG_ERR_NOMEM, "block factor row workspace");
-	BSG_CUDA(cudaMallocAsync(&A.big_owner, sizeof(int) * (BIG_SLOTS + 1), st));
+	BSG_CUDA(cudaMallocAsync(&A.big_owner, sizeof(int) * (BIG_SLOTS + 2), st));
 	A.nhold = A.big_owner + BIG_SLOTS;
+	A.nbig = A.nhold + 1;
 	A.hold_max = grid * FACT_WARPS_BLK / 2;
 	BSG_CUDA(cudaMallocAsync(&A.stats, sizeof(unsigned long long) * FACT_NSTAT, st));
 	// The pool first holds 8 blocks per block of A (block IC2 / ILU2 keep
@@ -1881,7 +2165,7 @@ int bsg_bfact_dyn(bsg_ctx *c, int nb, int sym, const bsg_param *p, const int *bi
 		BSG_CUDA(cudaMemsetAsync(qhead, 0, sizeof(unsigned long long), st));
 		BSG_CUDA(cudaMemsetAsync(qtail, 0, sizeof(unsigned long long), st));
 		BSG_CUDA(cudaMemsetAsync(done_count, 0, sizeof(int), st));
-		BSG_CUDA(cudaMemsetAsync(A.big_owner, 0, sizeof(int) * (BIG_SLOTS + 1), st));
+		BSG_CUDA(cudaMemsetAsync(A.big_owner, 0, sizeof(int) * (BIG_SLOTS + 2), st));
 		BSG_CUDA(cudaMemsetAsync(A.stats, 0, sizeof(unsigned long long) * FACT_NSTAT, st));
 		BSG_COUNT(4);
 		k_fact_init<<<nb_blocks(nb), 256, 0, st>>>(nb, it, nstat, whead, rec, acc, lev, inprog, c->d_stat);
