@@ -443,7 +443,8 @@ void bs_launch(cudaStream_t s, const bsg_bsell *m, int g, int k, long long ld, i
 template <typename VT>
 void bs_pass(cudaStream_t s, const bsg_bsell *m, int g, int k, long long ld, int ri, int ro, bool lin, bool lout,
              const double *d, const double *x, const double *yin, double *yout) {
-	if (k == 1) bs_launch<VT, 1, false, false>(s, m, g, k, ld, 0, 0, d, x, yin, yout);
+	// (a single vector left over from groups of 8 is interleaved like the others)
+	if (k == 1 && !lin) bs_launch<VT, 1, false, false>(s, m, g, k, ld, 0, 0, d, x, yin, yout);
 	else if (lin && lout) {
 		if (k <= 4) bs_launch<VT, 4, true, true>(s, m, g, k, ld, ri, ro, d, x, yin, yout);
 		else bs_launch<VT, 8, true, true>(s, m, g, k, ld, ri, ro, d, x, yin, yout);
