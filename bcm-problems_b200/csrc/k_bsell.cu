@@ -25,6 +25,7 @@
 #include "bsg_internal.cuh"
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
+#include <type_traits>
 
 #define BS_C 8
 #define BS_LONG 64
@@ -305,6 +306,107 @@ __global__ void __launch_bounds__(256, 1) k_bsell_sweep(int nb, int nr, long lon
 	}
 }
 
+// The same pass for systems too small to fill the GPU with a lane per block row
+// (see bs_small): several lanes share a row, each with its own sums, so every
+// sum keeps its order and its bits.  One vector: lanes 0..2 of a
+// group of 4 hold a point row each (a third of the values, one sum).  Several
+// vectors: lane q of a group of G holds vector q (the lanes of a group read the
+// same values, one transaction).  Bound: a lane's chain of column load and
+// gather, so as many blocks as registers allow are in flight.
+template <typename VT, int G, bool LIN, bool LOUT>
+__global__ void __launch_bounds__(256) k_bsell_sweep_small(int nb, int nr, long long ld, int ri, int ro,
+                                                           const long long *__restrict__ off,
+                                                           const int *__restrict__ col, const VT *__restrict__ val,
+                                                           const double *__restrict__ d, const double *__restrict__ x,
+                                                           const double *__restrict__ yin, double *__restrict__ yout,
+                                                           bs_long<VT> lg) {
+	constexpr bool ONE = G == 1;              // one vector
+	constexpr int NQ = ONE ? 1 : 2;           // vectors of a long row's warp
+	const int lane = threadIdx.x & 31;
+	const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	const int nwarps = (gridDim.x * blockDim.x) >> 5;
+	const int parts = (nr + NQ - 1) / NQ;
+	if (lg.nlong) { // a block or warp per long row and pair of vectors
+		__shared__ double red[3 * NQ][8];
+		double s[NQ][3];
+		auto out = [&](int r, int q0) {
+#pragma unroll
+			for (int q = 0; q < NQ; q++)
+				if (q0 + q < nr)
+					bs_out(r, (q0 + q) * ld + 3 * (long long)r,
+					       LOUT ? (long long)r * ro + 3 * (q0 + q) : (q0 + q) * ld + 3 * (long long)r, d, x, s[q], yout);
+		};
+		for (int e = blockIdx.x; e < lg.nvlong * parts; e += gridDim.x) {
+			const int i = e / parts, q0 = NQ * (e % parts);
+			bs_long_sum<VT, true, NQ, LIN>(__ldg(lg.off + i), __ldg(lg.off + i + 1), threadIdx.x, nr - q0, ld, ri, lg.col,
+			                               lg.val, yin + (LIN ? 3LL * q0 : q0 * ld), red, s);
+			if (threadIdx.x == 0) out(__ldg(lg.row + i), q0);
+		}
+		for (int e = gw; e < (lg.nlong - lg.nvlong) * parts; e += nwarps) {
+			const int i = lg.nvlong + e / parts, q0 = NQ * (e % parts);
+			bs_long_sum<VT, false, NQ, LIN>(__ldg(lg.off + i), __ldg(lg.off + i + 1), lane, nr - q0, ld, ri, lg.col, lg.val,
+			                                yin + (LIN ? 3LL * q0 : q0 * ld), nullptr, s);
+			if (lane == 0) out(__ldg(lg.row + i), q0);
+		}
+	}
+	constexpr int GL = ONE ? 4 : G, RPW = 32 / GL, U = ONE ? 8 : 4;
+	const int part = lane % GL; // point row (one vector) or vector
+	for (int r0 = gw * RPW; r0 < nb; r0 += nwarps * RPW) {
+		const int i = r0 + lane / GL, slice = i / BS_C, l = i % BS_C;
+		const bool mine = i < nb && (ONE ? part < 3 : part < nr) && !(lg.mask && (__ldg(lg.mask + slice) >> l & 1u));
+		double s[3] = {0.0, 0.0, 0.0};
+		if (mine) {
+			const long long base = __ldg(off + slice);
+			const int w = (int)((__ldg(off + slice + 1) - base) / BS_C);
+			const int *cp = col + base + l;
+			const VT *vp = val + 9 * base + l + (ONE ? 3 * BS_C * part : 0);
+			const double *yp = ONE ? yin : yin + (LIN ? 3LL * part : part * ld);
+			const int rj = LIN ? ri : 3;
+			constexpr int NV = ONE ? 3 : 9; // values of a block this lane multiplies
+			auto blocks = [&](int k, auto n) {
+				constexpr int N = decltype(n)::value;
+				int J[N];
+				VT a[N][NV];
+				double y[N][3];
+#pragma unroll
+				for (int u = 0; u < N; u++) {
+					J[u] = __ldg(cp + BS_C * (k + u));
+#pragma unroll
+					for (int p = 0; p < NV; p++) a[u][p] = __ldg(vp + 72LL * (k + u) + BS_C * p);
+				}
+#pragma unroll
+				for (int u = 0; u < N; u++)
+#pragma unroll
+					for (int c = 0; c < 3; c++) y[u][c] = __ldg(yp + (long long)J[u] * rj + c);
+#pragma unroll
+				for (int u = 0; u < N; u++) {
+					if (ONE) {
+#pragma unroll
+						for (int c = 0; c < 3; c++) s[0] = fma((double)a[u][c], y[u][c], s[0]);
+					} else {
+						bs_acc(a[u], y[u][0], y[u][1], y[u][2], s);
+					}
+				}
+			};
+			int k = 0;
+			for (; k + U <= w; k += U) blocks(k, std::integral_constant<int, U>());
+			for (; k < w; k++) blocks(k, std::integral_constant<int, 1>());
+		}
+		if (ONE) { // y_r = row r of D times the three differences
+			const double t = mine ? x[3 * (long long)i + part] - s[0] : 0.0;
+			const double t0 = __shfl_sync(0xffffffffu, t, 0, 4), t1 = __shfl_sync(0xffffffffu, t, 1, 4),
+			             t2 = __shfl_sync(0xffffffffu, t, 2, 4);
+			if (mine) {
+				const double *b = d + 9 * (size_t)i + part;
+				yout[3 * (long long)i + part] = fma(__ldg(b + 6), t2, fma(__ldg(b + 3), t1, __ldg(b) * t0));
+			}
+		} else if (mine) {
+			bs_out(i, part * ld + 3 * (long long)i, LOUT ? (long long)i * ro + 3 * part : part * ld + 3 * (long long)i, d, x,
+			       s, yout);
+		}
+	}
+}
+
 // y = D x for nr vectors, x at stride 3 nb, y at stride 3 nb or (ro > 0)
 // interleaved with row stride ro (the first Jacobi iterate)
 __global__ void k_bs_diag(int nb, int nr, int ro, const double *__restrict__ d, const double *__restrict__ x,
@@ -438,11 +540,45 @@ void bs_launch(cudaStream_t s, const bsg_bsell *m, int g, int k, long long ld, i
 	                                                             (const VT *)m->val, d, x, yin, yout, bs_long_of<VT>(m));
 }
 
+template <typename VT, int G, bool LIN, bool LOUT>
+void bs_launch_small(cudaStream_t s, const bsg_bsell *m, int k, long long ld, int ri, int ro, const double *d,
+                     const double *x, const double *yin, double *yout) {
+	const long long rows = 32 / (G == 1 ? 4 : G), parts = G == 1 ? 1 : (k + 1) / 2;
+	long long warps = (m->nb + rows - 1) / rows; // a warp's work either way
+	if ((m->nlong - m->nvlong) * parts > warps) warps = (m->nlong - m->nvlong) * parts;
+	if (m->nvlong * parts * 8 > warps) warps = m->nvlong * parts * 8;
+	k_bsell_sweep_small<VT, G, LIN, LOUT><<<capped(warps, 8), 256, 0, s>>>(
+		m->nb, k, ld, ri, ro, m->off, m->col, (const VT *)m->val, d, x, yin, yout, bs_long_of<VT>(m));
+}
+
+// Block rows up to which several lanes share a row: there a pass waits on its few
+// warps, above it the extra loads of the values cost more than the warps gain.
+// us a pass, a lane a row / shared (Q1 elasticity on n^3 nodes, about 48 blocks a
+// row), FP64 one vector: 8000 rows 30 / 25, 22000 38 / 45; FP64 six vectors: 8000
+// 82 / 28, 22000 89 / 68, 39000 94 / 107; FP32 one vector: 39000 42 / 38, 64000
+// 49 / 63; FP32 six vectors: 39000 93 / 84, 64000 108 / 130.  The periodic cell
+// of 8000 rows (64 blocks a row, long rows among them): FP64 six vectors 134 / 37.
+bool bs_small(const bsg_bsell *m, int nr) { return m->nb <= (m->fp32 ? 40000 : nr == 1 ? 12000 : 24000); }
+
 // One pass over k vectors of a group; lin / lout pick the interleaved layouts
 // (several vectors only).
 template <typename VT>
 void bs_pass(cudaStream_t s, const bsg_bsell *m, int g, int k, long long ld, int ri, int ro, bool lin, bool lout,
              const double *d, const double *x, const double *yin, double *yout) {
+	if (bs_small(m, k)) {
+		if (k == 1 && !lin) bs_launch_small<VT, 1, false, false>(s, m, k, ld, 0, 0, d, x, yin, yout);
+		else if (lin && lout) {
+			if (k <= 4) bs_launch_small<VT, 4, true, true>(s, m, k, ld, ri, ro, d, x, yin, yout);
+			else bs_launch_small<VT, 8, true, true>(s, m, k, ld, ri, ro, d, x, yin, yout);
+		} else if (lin) {
+			if (k <= 4) bs_launch_small<VT, 4, true, false>(s, m, k, ld, ri, 0, d, x, yin, yout);
+			else bs_launch_small<VT, 8, true, false>(s, m, k, ld, ri, 0, d, x, yin, yout);
+		} else {
+			if (k <= 4) bs_launch_small<VT, 4, false, false>(s, m, k, ld, 0, 0, d, x, yin, yout);
+			else bs_launch_small<VT, 8, false, false>(s, m, k, ld, 0, 0, d, x, yin, yout);
+		}
+		return;
+	}
 	// (a single vector left over from groups of 8 is interleaved like the others)
 	if (k == 1 && !lin) bs_launch<VT, 1, false, false>(s, m, g, k, ld, 0, 0, d, x, yin, yout);
 	else if (lin && lout) {
