@@ -16,6 +16,7 @@
 //     read once for all of them.
 #include "bsg_internal.cuh"
 #include "k_stream.cuh"
+#include <type_traits>
 
 namespace {
 
@@ -141,6 +142,113 @@ __global__ void __launch_bounds__(256, K > 4 ? 4 : (K > 2 ? 5 : 8)) k_spmv_bsr3(
 	}
 }
 
+#define IL_R 6 // vectors side by side in the interleaved product
+
+// The vectors of a product side by side: out[i IL_R + q] = X[q ld + i], q < nr, 0 beyond.
+__global__ void __launch_bounds__(256) k_interleave(int n, int nr, const double *__restrict__ X, long long ld,
+                                                    double *__restrict__ out) {
+	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+		double v[IL_R];
+#pragma unroll
+		for (int q = 0; q < IL_R; q++) v[q] = q < nr ? X[q * ld + i] : 0.0;
+#pragma unroll
+		for (int q = 0; q < IL_R; q += 2)
+			*reinterpret_cast<double2 *>(out + (long long)i * IL_R + q) = make_double2(v[q], v[q + 1]);
+	}
+}
+
+// k_spmv_bsr3 for five or six vectors that lie side by side (k_interleave): there
+// a block's x is 18 contiguous doubles instead of six pieces of 24 bytes, one line
+// or two per block instead of six.  Bound of the strided form: the cache lines its
+// gathers touch (21 per 3 blocks; here about 14, values included).  Lane 9 t + 3 c
+// + p holds block t of three, column c and the vectors 2 p and 2 p + 1 with their
+// three row sums, so that x comes in one 16-byte load and is used three times.  The
+// partial sums and the order they are added in are those of k_spmv_bsr3: the same
+// bits.  us for six vectors, interleaving included, before / now: 68000 block rows
+// of 26 blocks 115 / 66, 216000 358 / 185, 22000 44 / 26, 8000 21 / 15, 2700 9 / 11
+// (not taken there).  For four vectors (69 / 69) and eight (122 / 123), whose lanes
+// do not fill the warp, the strided form stays.
+__global__ void __launch_bounds__(256, 4) k_spmv_bsr3_il(int nb, int nr, const int *__restrict__ ia,
+                                                         const int *__restrict__ ja, const double *__restrict__ a,
+                                                         const double *__restrict__ XI, double *__restrict__ Y,
+                                                         long long ld) {
+	constexpr int U = 4;
+	const int lane = threadIdx.x & 31;
+	const int t = lane / 9, c = lane % 9 / 3, p = lane % 3;
+	const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	const int nwarps = (gridDim.x * blockDim.x) >> 5;
+	const double *xp = XI + c * IL_R + 2 * p;
+	for (int br = warp; br < nb; br += nwarps) {
+		const int b = __ldg(ia + br), e = lane < 27 ? __ldg(ia + br + 1) : b;
+		double s[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+		auto step = [&](int j, auto n) {
+			constexpr int N = decltype(n)::value;
+			int J[N];
+			double v[N][3];
+			double2 x[N];
+#pragma unroll
+			for (int u = 0; u < N; u++) {
+				J[u] = __ldg(ja + j + 3 * u);
+#pragma unroll
+				for (int r = 0; r < 3; r++) v[u][r] = __ldg(a + 9LL * (j + 3 * u) + 3 * r + c);
+			}
+#pragma unroll
+			for (int u = 0; u < N; u++) x[u] = __ldg(reinterpret_cast<const double2 *>(xp + 3LL * IL_R * J[u]));
+#pragma unroll
+			for (int u = 0; u < N; u++)
+#pragma unroll
+				for (int r = 0; r < 3; r++) {
+					s[r][0] = fma(v[u][r], x[u].x, s[r][0]);
+					s[r][1] = fma(v[u][r], x[u].y, s[r][1]);
+				}
+		};
+		int j = b + t;
+		for (; j + 3 * (U - 1) < e; j += 3 * U) step(j, std::integral_constant<int, U>());
+		for (; j < e; j += 3) step(j, std::integral_constant<int, 1>());
+#pragma unroll
+		for (int r = 0; r < 3; r++)
+#pragma unroll
+			for (int q = 0; q < 2; q++) {
+				double v = s[r][q] + __shfl_down_sync(0xffffffffu, s[r][q], 3);
+				v += __shfl_down_sync(0xffffffffu, s[r][q], 6);
+				double u = v + __shfl_down_sync(0xffffffffu, v, 9);
+				u += __shfl_down_sync(0xffffffffu, v, 18);
+				if (lane < 3 && 2 * p + q < nr) Y[(2 * p + q) * ld + 3LL * br + r] = u;
+			}
+	}
+}
+
+// Whether products of five or six vectors go interleaved: enough rows to pay for
+// the interleaving, and no capture going on (the workspace comes from the
+// stream's pool).
+bool bsr3_il_applies(const bsg_mat *m, cudaStream_t s) {
+	if (m->n < 6000) return false;
+	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+		cudaGetLastError();
+		return false;
+	}
+	return cs == cudaStreamCaptureStatusNone;
+}
+
+// The interleaved product of nr <= 6 vectors; 1 when there is no memory for it.
+int bsr3_interleaved(const bsg_mat *m, int nr, const double *X, double *Y, long long ld, cudaStream_t s) {
+	const int n = 3 * m->n;
+	double *xi = nullptr;
+	if (cudaMallocAsync(&xi, sizeof(double) * (size_t)n * IL_R, s) != cudaSuccess) {
+		cudaGetLastError();
+		return 1;
+	}
+	BSG_COUNT(2);
+	const int gi = (n + 255) / 256 < BSG_SMS * 8 ? (n + 255) / 256 : BSG_SMS * 8;
+	k_interleave<<<gi, 256, 0, s>>>(n, nr, X, ld, xi);
+	const int g = (m->n + 7) / 8 < BSG_SMS * 4 ? (m->n + 7) / 8 : BSG_SMS * 4; // resident blocks: 4 per SM (launch bounds)
+	k_spmv_bsr3_il<<<g, 256, 0, s>>>(m->n, nr, m->d_ia, m->d_ja, m->d_a, xi, Y, ld);
+	const cudaError_t e = cudaGetLastError();
+	cudaFreeAsync(xi, s);
+	return e == cudaSuccess ? BSG_OK : BSG_ERR_CUDA;
+}
+
 template <int K>
 int bsr3_grid(int nb) {
 	static int cap = 0;
@@ -170,11 +278,20 @@ int bsg_choose_group(double mean_row) {
 
 int bsg_spmm_launch(const bsg_mat *m, int nrhs, const double *X, double *Y, long long ld, cudaStream_t s) {
 	if (m->bs == 3) {
-		for (int r0 = 0; r0 < nrhs; r0 += 8) {
-			BSG_COUNT(1);
-			const int k = nrhs - r0 < 8 ? nrhs - r0 : 8;
+		const bool il = nrhs >= 5 && bsr3_il_applies(m, s);
+		int k;
+		for (int r0 = 0; r0 < nrhs; r0 += k) {
+			// groups of 8 vectors; of 6 while more than 8 are left and they go
+			// interleaved (us, 68000 block rows: 6 + 5 vectors 132, 8 + 3 187)
+			k = nrhs - r0 <= 8 ? nrhs - r0 : il ? IL_R : 8;
 			const double *Xr = X + r0 * ld;
 			double *Yr = Y + r0 * ld;
+			if (il && (k == 5 || k == 6)) {
+				const int rc = bsr3_interleaved(m, k, Xr, Yr, ld, s);
+				if (rc == BSG_OK) continue;
+				if (rc < 0) return rc;
+			}
+			BSG_COUNT(1);
 			if (k == 1) k_spmv_bsr3<1><<<bsr3_grid<1>(m->n), 256, 0, s>>>(m->n, k, m->d_ia, m->d_ja, m->d_a, Xr, Yr, ld);
 			else if (k == 2) k_spmv_bsr3<2><<<bsr3_grid<2>(m->n), 256, 0, s>>>(m->n, k, m->d_ia, m->d_ja, m->d_a, Xr, Yr, ld);
 			else if (k <= 4) k_spmv_bsr3<4><<<bsr3_grid<4>(m->n), 256, 0, s>>>(m->n, k, m->d_ia, m->d_ja, m->d_a, Xr, Yr, ld);
