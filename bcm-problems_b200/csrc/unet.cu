@@ -194,6 +194,122 @@ __global__ void __launch_bounds__(128) k_conv3(ConvArgs a) {
 	}
 }
 
+// k_conv3 for grids with few tiles: 16 MT voxels x 16 output channels a CTA, and the
+// weights come from L2 as fragments, S steps of 16 input channels in flight at
+// once, where k_conv3 first stages a slice of up to 117 KB that a tile or two
+// then use.  Bound: the latency of those loads, and with many CTAs their number
+// (MT tiles share the weights).  The taps a warp takes, the order of its MMAs and
+// of the warps' partial sums are k_conv3's: the same bits.  us of a whole forward
+// pass, k_conv3 / this: 16^3 155 / 107, 64^3 257 / 214, 96x64x32 284 / 224, 128^3
+// (one level) 501 / 474; of a training sample 64^3 702 / 605.  MT kept so that two
+// CTAs a SM remain (one: 64^3 221, four: 217); more than 100000 voxels x 16-channel
+// slices go to k_conv3 (80x72x64: 674 with the limit, 700 without).
+#define CONV_FEW 6250 // 16-voxel tiles x slices
+#define FEW_CTAS (2 * BSG_SMS)
+template <bool F32OUT, int MT, int S>
+__global__ void __launch_bounds__(128) k_conv3_few(ConvArgs a, int lgcb) {
+	__shared__ float red[3][MT * 8][32];
+	const int Cin = a.Ca + a.Cb;
+	const int slice = blockIdx.y; // 16 output channels
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int g = lane >> 2, t4 = lane & 3;
+	const long long nvox = (long long)a.nz * a.ny * a.nx;
+	const int nyA = a.ny >> a.upA, nxA = a.nx >> a.upA;
+	// rows of this lane: voxels g and g + 8 of each tile
+	int vz[MT][2], vy[MT][2], vx[MT][2];
+#pragma unroll
+	for (int m = 0; m < MT; m++)
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			const long long v = (blockIdx.x * (long long)MT + m) * 16 + g + 8 * h;
+			vx[m][h] = (int)(v % a.nx);
+			vy[m][h] = (int)((v / a.nx) % a.ny);
+			vz[m][h] = v < nvox ? (int)(v / ((long long)a.nx * a.ny)) : -8; // beyond the grid: every tap outside
+		}
+	float acc[MT][2][4];
+#pragma unroll
+	for (int m = 0; m < MT; m++)
+#pragma unroll
+		for (int j = 0; j < 2; j++)
+#pragma unroll
+			for (int q = 0; q < 4; q++) acc[m][j][q] = 0.f;
+	const bf16 *wl = a.W + (size_t)(slice * 16 + g) * Cin + 2 * t4; // rows g (and g + 8) of the slice
+	// steps of this warp: taps warp, warp + 4, .., each over the 2^lgcb groups of 16 input channels
+	const int steps = ((27 - warp + 3) / 4) << lgcb;
+	for (int s0 = 0; s0 < steps; s0 += S) {
+		unsigned af[S][MT][4], b[S][2][2];
+#pragma unroll
+		for (int u = 0; u < S; u++) {
+			const int s = min(s0 + u, steps - 1);
+			const int tap = warp + 4 * (s >> lgcb), cb = 16 * (s & ((1 << lgcb) - 1));
+			const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
+			const bf16 *wr = wl + (size_t)tap * a.Cout * Cin + cb;
+#pragma unroll
+			for (int j = 0; j < 2; j++) {
+				b[u][j][0] = ld_u32(wr + (size_t)(8 * j) * Cin);
+				b[u][j][1] = ld_u32(wr + (size_t)(8 * j) * Cin + 8);
+			}
+			const bool fromA = cb < a.Ca;
+#pragma unroll
+			for (int m = 0; m < MT; m++)
+#pragma unroll
+				for (int h = 0; h < 2; h++) {
+					const int z = vz[m][h] + dz, y = vy[m][h] + dy, x = vx[m][h] + dx;
+					af[u][m][h] = af[u][m][2 + h] = 0u;
+					if (z >= 0 && z < a.nz && y >= 0 && y < a.ny && x >= 0 && x < a.nx) {
+						const bf16 *src =
+							fromA ? a.A + (((long long)(z >> a.upA) * nyA + (y >> a.upA)) * nxA + (x >> a.upA)) * a.Ca + cb
+							      : a.B + (((long long)z * a.ny + y) * a.nx + x) * a.Cb + (cb - a.Ca);
+						af[u][m][h] = ld_u32(src + 2 * t4);
+						af[u][m][2 + h] = ld_u32(src + 2 * t4 + 8);
+					}
+				}
+		}
+#pragma unroll
+		for (int u = 0; u < S; u++)
+			if (s0 + u < steps)
+#pragma unroll
+				for (int m = 0; m < MT; m++)
+#pragma unroll
+					for (int j = 0; j < 2; j++) mma_bf16(acc[m][j], af[u][m], b[u][j][0], b[u][j][1]);
+	}
+	// warps 1-3 hand their partial sums to warp 0
+	if (warp > 0)
+#pragma unroll
+		for (int m = 0; m < MT; m++)
+#pragma unroll
+			for (int j = 0; j < 2; j++)
+#pragma unroll
+				for (int q = 0; q < 4; q++) red[warp - 1][(m * 2 + j) * 4 + q][lane] = acc[m][j][q];
+	__syncthreads();
+	if (warp > 0) return;
+#pragma unroll
+	for (int w = 0; w < 3; w++)
+#pragma unroll
+		for (int m = 0; m < MT; m++)
+#pragma unroll
+			for (int j = 0; j < 2; j++)
+#pragma unroll
+				for (int q = 0; q < 4; q++) acc[m][j][q] += red[w][(m * 2 + j) * 4 + q][lane];
+#pragma unroll
+	for (int m = 0; m < MT; m++)
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			const long long v = (blockIdx.x * (long long)MT + m) * 16 + g + 8 * h;
+			if (v >= nvox) continue;
+#pragma unroll
+			for (int j = 0; j < 2; j++) {
+				const int co = slice * 16 + j * 8 + 2 * t4;
+				const float c0 = acc[m][j][2 * h], c1 = acc[m][j][2 * h + 1];
+				if (F32OUT)
+					*reinterpret_cast<float2 *>(static_cast<float *>(a.out) + v * a.Cout + co) = make_float2(c0, c1);
+				else
+					*reinterpret_cast<__nv_bfloat162 *>(static_cast<bf16 *>(a.out) + v * a.Cout + co) =
+					    __floats2bfloat162_rn(fmaxf(c0, 0.f), fmaxf(c1, 0.f));
+			}
+		}
+}
+
 // ---- shared-memory tiled convolution (grids with nx % 32 == 0) ------------
 // A CTA (8 warps) computes a 32 x 4 x 2 brick of output voxels for 16 output
 // channels.  Input channels go in chunks of CH (16 or 32): the CTA stages the
@@ -1342,6 +1458,20 @@ int conv_launch(bsg_unet *u, int lvl, const bf16 *A, int Ca, int upA, const bf16
 		else
 			rc = f32out ? conv_tiled<true, 16>(a, s) : conv_tiled<false, 16>(a, s);
 		if (rc) return rc;
+		BSG_CUDA(cudaGetLastError());
+		return BSG_OK;
+	}
+	const long long tiles = (u->nv[lvl] + 15) / 16 * (Cout / 16);
+	int lgcb = 0;
+	while ((16 << lgcb) < Cin) lgcb++;
+	if (tiles <= CONV_FEW && (16 << lgcb) == Cin) {
+		auto go = [&](auto kern, int mt) {
+			kern<<<dim3((unsigned)((u->nv[lvl] + 16 * mt - 1) / (16 * mt)), Cout / 16), 128, 0, s>>>(a, lgcb);
+		};
+		// as many tiles a CTA as still leave FEW_CTAS CTAs
+		if (tiles >= 4 * FEW_CTAS) f32out ? go(k_conv3_few<true, 4, 2>, 4) : go(k_conv3_few<false, 4, 2>, 4);
+		else if (tiles >= 2 * FEW_CTAS) f32out ? go(k_conv3_few<true, 2, 4>, 2) : go(k_conv3_few<false, 2, 4>, 2);
+		else f32out ? go(k_conv3_few<true, 1, 8>, 1) : go(k_conv3_few<false, 1, 8>, 1);
 		BSG_CUDA(cudaGetLastError());
 		return BSG_OK;
 	}

@@ -169,7 +169,7 @@ def _backward_rounded(A, W, gy):
     return G
 
 
-def _sparse_case(nx, ny, nz):
+def _sparse_case(nx, ny, nz, backward=True):
     """Weights of +-1 in three places per output channel, an input of 0, +-1/4
     and +-1: every forward sum is exact in FP32, so the GPU's activations (and the
     masks of the backward pass) are the reference's."""
@@ -191,7 +191,7 @@ def _sparse_case(nx, ny, nz):
     logd = np.where(up, 1.0, -1.0).reshape(nz, ny, nx)
     x0, _ = U.make_input(r.reshape(nz, ny, nx), logd)
     A = U.forward(x0, W)
-    want = _backward_rounded(A, W, U.loss(A["y"], t.reshape(nz, ny, nx))[1])
+    want = _backward_rounded(A, W, U.loss(A["y"], t.reshape(nz, ny, nx))[1]) if backward else None
     return W, r, t, np.where(up, np.exp(1.0), np.exp(-1.0)), A, want
 
 
@@ -213,4 +213,23 @@ def test_unet_gradients_on_ragged_grids(ctx, nx, ny, nz):
     for k in want:
         err = np.linalg.norm(G[k] - want[k])
         assert err <= 2.0 ** -8 * np.linalg.norm(want[k]), (k, err)
+    net.free()
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(8, 8, 8), (16, 24, 8), (24, 16, 40), (40, 48, 32), (104, 64, 40)])
+def test_unet_forward_on_ragged_grids(ctx, nx, ny, nz):
+    """Forward passes whose levels take one, two and four tiles a CTA, tiles that
+    run over the end of the grid among them.  The activations are exact (see
+    _sparse_case), the output is their 16-term FP32 sum: 16 roundings of 2^-24."""
+    import bsg
+    import torch
+    W, r, _, d, A, _ = _sparse_case(nx, ny, nz, backward=False)
+    net = bsg.UNet(ctx, nx, ny, nz)
+    net.set_weights(_flat(W))
+    net.set_diag(torch.as_tensor(d, device="cuda"))
+    y = torch.empty(nx * ny * nz, dtype=torch.float64, device="cuda")
+    net.forward(torch.as_tensor(r, device="cuda"), y)
+    scale = np.abs(A["d0"]) @ np.abs(W["w7"])
+    assert scale.max() > 0
+    assert np.all(np.abs(y.cpu().numpy().reshape(A["y"].shape) - A["y"]) <= 16 * 2.0 ** -24 * scale)
     net.free()
