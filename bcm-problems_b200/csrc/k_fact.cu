@@ -63,11 +63,27 @@
 #ifndef FACT_MINB
 #define FACT_MINB 2 // blocks per SM the registers must allow
 #endif
-#define CMAX 128   // members of C(i)
+// Capacities of the shared workspace.  A row that does not fit starts again in
+// global memory and keeps one of few workspaces while it waits, so a factor
+// where a few percent of the rows do is many times slower.  192 members (IC2
+// 17 KB a warp, 12 warps an SM) instead of 128: ILU2 of the 28x21x24
+// convection matrix 50 -> 18 ms, 44x40x36 132 -> 37.5, IC2 128^3 164 -> 154;
+// 160 gives the same.  For every row 320 members and 512 columns would cost
+// large factors their warps (IC2 128^3 154 -> 254 ms), so only a factor whose
+// rows overflow takes them (k_fact_rows<.., WIDE>): the kernel gives up, in
+// the first half of the rows, once more than WIDE_MIN + done / WIDE_DIV rows
+// did, and the factor starts again with the wide one (IC2, tau 2e-4, 24^3:
+// 293 -> 89 ms; a divisor of 16 gives 95, of 8 118, of 4 150; no factor whose
+// rows fit takes the wide kernel).  The factor does not depend on the
+// schedule, so both give the same bits.
+#define CMAX 192   // members of C(i)
 #define HCAP 256   // distinct mask columns per row (power of two)
-#ifndef PFCAP
 #define PFCAP 256  // prefetched contributor entries per row
-#endif
+#define CMAX_WIDE 320
+#define HCAP_WIDE 512
+#define FACT_WARPS_WIDE 2
+#define WIDE_MIN 64
+#define WIDE_DIV 32
 // capacities of the global-memory workspaces that take the rows that do not
 // fit the shared one (about 0.7 MB each), and how many there are
 #define BIG_SLOTS 64
@@ -82,16 +98,21 @@
 #ifndef WSETCAP
 #define WSETCAP 128 // far members (hash slots, a power of two)
 #endif
-// block rows (3 x 3 blocks): mask columns of the shared workspace, member
-// bitmap window
-#define HCAP_BLK 256
-#define CMAX_BLK 256
+// block rows (3 x 3 blocks): mask columns and members of the shared
+// workspace, member bitmap window.  512 of each leave room for one CTA of two
+// warps on an SM and still pay, since rows in global memory hold up all others
+// (256 of each -> 512: periodic IC2 of 20^3 block rows 326 -> 206 ms, 12^3
+// 104 -> 64, clamped 44^3 150 -> 134, ILU2 20^3 64 -> 54, 36^3 125 -> 110).
+// 1024 columns, or three warps, give no more.
+#define HCAP_BLK 512
+#define CMAX_BLK 512
 #define MWIN_BLK 8192
 #define FACT_WARPS_BLK 2 // warps of a CTA in block mode (larger workspaces)
 #define W_EMPTY (-1)
 #define W_CLOSED (-2)
 
 // row record: bit 63 done | bits 32..62 pool offset | bits 0..15 stored length
+#define SITE_WIDE 9 // BSG_ERR_WORKSPACE there: the factor wants the wide kernel
 #define REC_DONE (1ull << 63)
 #define REC_OFF(r) ((long long)(((r) >> 32) & 0x7fffffffull))
 #define REC_LEN(r) ((int)((r) & 0xffffull))
@@ -125,6 +146,7 @@ struct FactArgs {
 	int *big_owner;            // 1 while a warp holds that workspace
 	int *nhold;                // warps holding their row for a member nobody computes
 	int *nbig;                 // workspaces taken
+	int *novf;                 // rows that took one so far, without those of A's longest rows
 	int hold_max;              // at most this many (half the warps)
 };
 
@@ -146,11 +168,12 @@ struct PhaseClock {
 // U-side arrays, so more warps fit on an SM.  Block rows (BLK) keep 9
 // values per column (U side; ILU: then the L side at 9 (hcap + slot)) in hl
 // and read their members' blocks straight from the pool.
-template <bool ILU, bool BLK = false>
+template <bool ILU, bool BLK = false, bool WIDE = false>
 struct SmemWS {
 	static constexpr bool big = false, ilu = ILU, blk = BLK;
-	static constexpr int cmax = BLK ? CMAX_BLK : CMAX, hcap = BLK ? HCAP_BLK : HCAP, pfcap = PFCAP,
-	                     wcap = WSETCAP, mwin = BLK ? MWIN_BLK : MWIN;
+	static constexpr int cmax = BLK ? CMAX_BLK : WIDE ? CMAX_WIDE : CMAX,
+	                     hcap = BLK ? HCAP_BLK : WIDE ? HCAP_WIDE : HCAP, pfcap = PFCAP, wcap = WSETCAP,
+	                     mwin = BLK ? MWIN_BLK : MWIN;
 	int W[cmax];           // members (discovery order, then sorted)
 	int Wp[cmax];          // pool index of column i in that row (stored members)
 	int We[cmax];          // pool end of that row
@@ -162,7 +185,7 @@ struct SmemWS {
 	int wset[WSETCAP];     // membership hash of W (keys), members below i - mwin
 	unsigned wbits[mwin > 0 ? mwin / 32 : 1]; // membership bitmap: bit i - 1 - k for member k
 	int hkey[hcap];        // column accumulator
-	double hl[BLK ? hcap * (ILU ? 18 : 9) : HCAP], hu[ILU && !BLK ? HCAP : 1];
+	double hl[BLK ? hcap * (ILU ? 18 : 9) : hcap], hu[ILU && !BLK ? hcap : 1];
 	int lsts[hcap];        // selected members (updates); sorted slots (finish)
 	// the updates' prefetch buffers and the finish's slot lists are never
 	// live at once; Wlv (depth of a closed member) lives in a closure pass
@@ -177,7 +200,8 @@ struct SmemWS {
 		};
 		int Wlv[cmax];
 	};
-	double pf_l[BLK ? 1 : PFCAP], pf_u[ILU && !BLK ? PFCAP : 1];
+	double pf_l[BLK ? 1 : hcap > PFCAP ? hcap : PFCAP]; // (the finish lists up to hcap compensations here)
+	double pf_u[ILU && !BLK ? PFCAP : 1];
 	int sc[4];
 	short slots[hcap];     // the accumulator slots in use, in insertion order (the diagonal first)
 	short srt[hcap];       // the off-diagonal ones among them by ascending column (see sort_columns)
@@ -1685,12 +1709,16 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 	return -1;
 }
 
-template <bool ILU, bool BLK>
-__global__ void __launch_bounds__((BLK ? FACT_WARPS_BLK : FACT_WARPS) * 32, FACT_MINB) k_fact_rows(FactArgs A) {
-	constexpr int fw = BLK ? FACT_WARPS_BLK : FACT_WARPS;
+// Warps of a CTA.
+template <bool BLK, bool WIDE>
+constexpr int fact_warps = BLK ? FACT_WARPS_BLK : WIDE ? FACT_WARPS_WIDE : FACT_WARPS;
+
+template <bool ILU, bool BLK, bool WIDE>
+__global__ void __launch_bounds__(fact_warps<BLK, WIDE> * 32, FACT_MINB) k_fact_rows(FactArgs A) {
+	constexpr int fw = fact_warps<BLK, WIDE>;
 	extern __shared__ unsigned char smem_raw[];
 	const int warp = threadIdx.x >> 5;
-	SmemWS<ILU, BLK> &s = reinterpret_cast<SmemWS<ILU, BLK> *>(smem_raw)[warp];
+	SmemWS<ILU, BLK, WIDE> &s = reinterpret_cast<SmemWS<ILU, BLK, WIDE> *>(smem_raw)[warp];
 	const int lane = threadIdx.x & 31;
 	PhaseClock pc;
 #pragma unroll
@@ -1729,7 +1757,16 @@ __global__ void __launch_bounds__((BLK ? FACT_WARPS_BLK : FACT_WARPS) * 32, FACT
 					const int q = (start + k) % BIG_SLOTS;
 					if (atomicCAS(A.big_owner + q, 0, 1) == 0) slot = q;
 				}
-				if (slot >= 0) atomicAdd(A.nbig, 1);
+				if (slot >= 0) {
+					atomicAdd(A.nbig, 1);
+					// (rows that A itself makes long are left out: the
+					// wide kernel need not take them either)
+					if (!BLK && !WIDE && A.iu[i + 1] - A.iu[i] < HCAP) {
+						const int novf = atomicAdd(A.novf, 1) + 1, done = *(volatile int *)A.done_count;
+						if (novf > WIDE_MIN + done / WIDE_DIV && done < A.n / 2)
+							devstat_fail(A.st, BSG_ERR_WORKSPACE, i, SITE_WIDE);
+					}
+				}
 			}
 			slot = __shfl_sync(0xffffffffu, slot, 0);
 			if (slot < 0) {
@@ -1966,18 +2003,12 @@ int bsg_fact_run(bsg_ctx *c, bsg_mat *m, int kind, const bsg_param *p, bsg_fct *
 	BSG_CUDA(cudaMallocAsync(&pool_len, sizeof(unsigned long long), st));
 	BSG_CUDA(cudaMallocAsync(&qhead, sizeof(unsigned long long), st));
 	BSG_CUDA(cudaMallocAsync(&qtail, sizeof(unsigned long long), st));
-	BSG_CUDA(cudaMemsetAsync(pool_len, 0, sizeof(unsigned long long), st));
-	BSG_CUDA(cudaMemsetAsync(qhead, 0, sizeof(unsigned long long), st));
-	BSG_CUDA(cudaMemsetAsync(qtail, 0, sizeof(unsigned long long), st));
-	BSG_CUDA(cudaMemsetAsync(done_count, 0, sizeof(int), st));
 	BSG_CUDA(cudaMemsetAsync(c->d_stat, 0, sizeof(bsg_devstat), st));
 
 	cudaEventRecord(c->ev0, st);
 	// scale, init, queue fill, seed, rows, count, emit (+ CUB scans)
 	BSG_COUNT(7);
 	k_fact_scale<<<nb(n, 256), 256, 0, st>>>(n, kind, m->d_iu, m->d_ju, m->d_al, p->sclmin, scll, sclu, diag0, c->d_stat);
-	k_fact_init<<<nb(n, 256), 256, 0, st>>>(n, m->d_it, nstat, whead, rec, acc, lev, inprog, c->d_stat);
-	k_fill_int<<<BSG_SMS * 4, 256, 0, st>>>(qcap, queue, -1);
 	FactArgs A;
 	A.n = n; A.kind = kind;
 	A.iu = m->d_iu; A.ju = m->d_ju; A.al = m->d_al; A.au = m->d_au;
@@ -1990,31 +2021,51 @@ int bsg_fact_run(bsg_ctx *c, bsg_mat *m, int kind, const bsg_param *p, bsg_fct *
 	A.nstat = nstat; A.whead = whead; A.wnext = wnext; A.inprog = inprog; A.queue = queue; A.qcap = qcap;
 	A.qhead = qhead; A.qtail = qtail; A.done_count = done_count; A.st = c->d_stat;
 	BSG_CUDA(cudaMallocAsync(&A.stats, sizeof(unsigned long long) * FACT_NSTAT, st));
-	BSG_CUDA(cudaMemsetAsync(A.stats, 0, sizeof(unsigned long long) * FACT_NSTAT, st));
-	k_fact_seed<<<nb(n, 256), 256, 0, st>>>(A);
-	void (*kern)(FactArgs) = kind == 1 ? k_fact_rows<true, false> : k_fact_rows<false, false>;
-	const size_t smem = (kind == 1 ? sizeof(SmemWS<true>) : sizeof(SmemWS<false>)) * FACT_WARPS;
-	BSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-	int per_sm = 0;
-	BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FACT_WARPS * 32, smem));
-	if (per_sm < 1) per_sm = 1;
-	int grid = per_sm * BSG_SMS;
-	int need = (n + FACT_WARPS - 1) / FACT_WARPS;
-	if (grid > need) grid = need;
-	if (grid < 1) grid = 1;
 	if (cudaMallocAsync(&A.big_ws, GlobWS<true>::bytes * (size_t)BIG_SLOTS, st) != cudaSuccess)
 		return bsg_set_error(BSG_ERR_NOMEM, "factor row workspace");
-	BSG_CUDA(cudaMallocAsync(&A.big_owner, sizeof(int) * (BIG_SLOTS + 2), st));
-	BSG_CUDA(cudaMemsetAsync(A.big_owner, 0, sizeof(int) * (BIG_SLOTS + 2), st));
+	BSG_CUDA(cudaMallocAsync(&A.big_owner, sizeof(int) * (BIG_SLOTS + 3), st));
 	A.nhold = A.big_owner + BIG_SLOTS;
 	A.nbig = A.nhold + 1;
-	A.hold_max = grid * FACT_WARPS / 2;
-	kern<<<grid, FACT_WARPS * 32, smem, st>>>(A);
-	BSG_CUDA(cudaGetLastError());
+	A.novf = A.nbig + 1;
+	int grid = 1, warps = FACT_WARPS;
+	for (bool wide = false;; wide = true) {
+		BSG_CUDA(cudaMemsetAsync(pool_len, 0, sizeof(unsigned long long), st));
+		BSG_CUDA(cudaMemsetAsync(qhead, 0, sizeof(unsigned long long), st));
+		BSG_CUDA(cudaMemsetAsync(qtail, 0, sizeof(unsigned long long), st));
+		BSG_CUDA(cudaMemsetAsync(done_count, 0, sizeof(int), st));
+		BSG_CUDA(cudaMemsetAsync(A.stats, 0, sizeof(unsigned long long) * FACT_NSTAT, st));
+		BSG_CUDA(cudaMemsetAsync(A.big_owner, 0, sizeof(int) * (BIG_SLOTS + 3), st));
+		k_fact_init<<<nb(n, 256), 256, 0, st>>>(n, m->d_it, nstat, whead, rec, acc, lev, inprog, c->d_stat);
+		k_fill_int<<<BSG_SMS * 4, 256, 0, st>>>(qcap, queue, -1);
+		k_fact_seed<<<nb(n, 256), 256, 0, st>>>(A);
+		void (*kern)(FactArgs) = kind == 1 ? (wide ? k_fact_rows<true, false, true> : k_fact_rows<true, false, false>)
+		                                   : (wide ? k_fact_rows<false, false, true> : k_fact_rows<false, false, false>);
+		warps = wide ? fact_warps<false, true> : fact_warps<false, false>;
+		const size_t ws = kind == 1 ? (wide ? sizeof(SmemWS<true, false, true>) : sizeof(SmemWS<true>))
+		                            : (wide ? sizeof(SmemWS<false, false, true>) : sizeof(SmemWS<false>));
+		const size_t smem = ws * warps;
+		BSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		int per_sm = 0;
+		BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem));
+		grid = (per_sm < 1 ? 1 : per_sm) * BSG_SMS;
+		const int need = (n + warps - 1) / warps;
+		if (grid > need) grid = need;
+		if (grid < 1) grid = 1;
+		A.hold_max = grid * warps / 2;
+		kern<<<grid, warps * 32, smem, st>>>(A);
+		BSG_CUDA(cudaGetLastError());
+		if (wide) break;
+		bsg_devstat h;
+		BSG_CUDA(cudaMemcpyAsync(&h, c->d_stat, sizeof(h), cudaMemcpyDeviceToHost, st));
+		BSG_CUDA(cudaStreamSynchronize(st));
+		if (h.code != BSG_ERR_WORKSPACE || h.pad[0] != SITE_WIDE) break;
+		BSG_CUDA(cudaMemsetAsync(c->d_stat, 0, sizeof(bsg_devstat), st));
+		BSG_COUNT(4);
+	}
 	int rc = bsg_check_devstat(c);
 	cudaMemcpyAsync(g_fact_stats, A.stats, sizeof(g_fact_stats), cudaMemcpyDeviceToHost, st);
 	cudaStreamSynchronize(st);
-	g_fact_stats[FS_WARPS] = (unsigned long long)grid * FACT_WARPS; // warps launched
+	g_fact_stats[FS_WARPS] = (unsigned long long)grid * warps; // warps launched
 	cudaFreeAsync(A.stats, st);
 	cudaFreeAsync(A.big_ws, st);
 	cudaFreeAsync(A.big_owner, st);
@@ -2119,7 +2170,7 @@ int bsg_bfact_dyn(bsg_ctx *c, int nb, int sym, const bsg_param *p, const int *bi
 	BSG_CUDA(cudaMallocAsync(&pool_len, sizeof(unsigned long long), st));
 	BSG_CUDA(cudaMallocAsync(&qhead, sizeof(unsigned long long), st));
 	BSG_CUDA(cudaMallocAsync(&qtail, sizeof(unsigned long long), st));
-	void (*kern)(FactArgs) = kind == 1 ? k_fact_rows<true, true> : k_fact_rows<false, true>;
+	void (*kern)(FactArgs) = kind == 1 ? k_fact_rows<true, true, false> : k_fact_rows<false, true, false>;
 	const size_t smem = (kind == 1 ? sizeof(SmemWS<true, true>) : sizeof(SmemWS<false, true>)) * FACT_WARPS_BLK;
 	const size_t big = kind == 1 ? GlobWS<true, true>::bytes : GlobWS<false, true>::bytes;
 	BSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2144,9 +2195,10 @@ int bsg_bfact_dyn(bsg_ctx *c, int nb, int sym, const bsg_param *p, const int *bi
 	A.qhead = qhead; A.qtail = qtail; A.done_count = done_count; A.st = c->d_stat;
 	if (cudaMallocAsync(&A.big_ws, big * (size_t)BIG_SLOTS, st) != cudaSuccess)
 		return bsg_set_error(BSG_ERR_NOMEM, "block factor row workspace");
-	BSG_CUDA(cudaMallocAsync(&A.big_owner, sizeof(int) * (BIG_SLOTS + 2), st));
+	BSG_CUDA(cudaMallocAsync(&A.big_owner, sizeof(int) * (BIG_SLOTS + 3), st));
 	A.nhold = A.big_owner + BIG_SLOTS;
 	A.nbig = A.nhold + 1;
+	A.novf = A.nbig + 1; // (not counted for block rows)
 	A.hold_max = grid * FACT_WARPS_BLK / 2;
 	BSG_CUDA(cudaMallocAsync(&A.stats, sizeof(unsigned long long) * FACT_NSTAT, st));
 	// The pool first holds 8 blocks per block of A (block IC2 / ILU2 keep
@@ -2165,7 +2217,7 @@ int bsg_bfact_dyn(bsg_ctx *c, int nb, int sym, const bsg_param *p, const int *bi
 		BSG_CUDA(cudaMemsetAsync(qhead, 0, sizeof(unsigned long long), st));
 		BSG_CUDA(cudaMemsetAsync(qtail, 0, sizeof(unsigned long long), st));
 		BSG_CUDA(cudaMemsetAsync(done_count, 0, sizeof(int), st));
-		BSG_CUDA(cudaMemsetAsync(A.big_owner, 0, sizeof(int) * (BIG_SLOTS + 2), st));
+		BSG_CUDA(cudaMemsetAsync(A.big_owner, 0, sizeof(int) * (BIG_SLOTS + 3), st));
 		BSG_CUDA(cudaMemsetAsync(A.stats, 0, sizeof(unsigned long long) * FACT_NSTAT, st));
 		BSG_COUNT(4);
 		k_fact_init<<<nb_blocks(nb), 256, 0, st>>>(nb, it, nstat, whead, rec, acc, lev, inprog, c->d_stat);
