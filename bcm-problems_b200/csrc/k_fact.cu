@@ -14,7 +14,7 @@
 // between m and i", and a member that does not store i has dropped it.
 //
 // Schedule (dynamic, deadlock-free).  A row enters a global FIFO queue when
-// every row of A's column i has been claimed by a warp and all but one or two
+// every row of A's column i has been claimed by a warp and all but a few
 // are finished (see Admission).  A warp pops a row and tries it: it builds C(i) over
 // finished rows (one member per lane, rows read with 16-byte loads).  An
 // unfinished member m that another warp is computing is waited for; a member
@@ -499,12 +499,16 @@ __device__ __forceinline__ long long q_backlog(const FactArgs &A) {
 // 15..29); bit 30 marks j queued once, bit 31 claimed once.  Row j enters the
 // queue when all of them are claimed and at most one is unfinished: it then
 // starts while its last predecessor is being computed and waits for it.  With
-// more than a sixteenth of the warps idle it enters with two unfinished: a row
-// takes tens of microseconds before its first wait, and one that starts late
-// holds up its chain; not while the global workspaces are in demand, where a
-// waiting row keeps one from the rows it waits for (IC2 32^3 18.2 -> 12.3 ms, 80x72x65 66.7 -> 54.4; always
-// with two unfinished, waiting rows take the warps that others need: 80x72x65
-// 206 ms, 128^3 1.3 s).  A row that another row waits for is queued earlier
+// more than a sixteenth of the warps idle it enters with two unfinished, with
+// more than half of them idle with up to four: a row takes tens of microseconds
+// before its first wait (a block row hundreds), and one that starts late holds
+// up its chain; not while the global workspaces are in demand, where a waiting
+// row keeps one from the rows it waits for.  Never -> two -> up to four: IC2
+// 32^3 18.2 -> 12.2 -> 11.1 ms, with thresholds 1e-2 and 1e-4 30.7 (two) ->
+// 25.2, 80x72x65 66.7 -> 49.7 -> 49.7, block IC2 periodic 20^3 210 (two) -> 185,
+// 12^3 64 -> 48, ILU2 20^3 54 -> 42.5; up to eight: 174, 39 and 48.  (Always with
+// two unfinished, waiting rows take the warps that others need: 80x72x65
+// 206 ms, 128^3 1.3 s.)  A row that another row waits for is queued earlier
 // (promoted) if nobody has queued it yet.  Bit 30 makes the first of these the
 // only one: a row is queued once this way, and again only when a row it parked
 // on finishes.
@@ -512,11 +516,8 @@ __device__ __forceinline__ long long q_backlog(const FactArgs &A) {
 #define ADM_ONE_CLAIM (1u << 15)
 #define ADM_QUEUED (1u << 30)
 #define ADM_CLAIMED (1u << 31)
-#ifndef BSG_ADMIT_UNFINISHED
-#define BSG_ADMIT_UNFINISHED 1
-#endif
 __device__ __forceinline__ bool admissible(unsigned v) {
-	return ((v >> 15) & 0x7fffu) == 0 && (v & 0x7fffu) <= BSG_ADMIT_UNFINISHED;
+	return ((v >> 15) & 0x7fffu) == 0 && (v & 0x7fffu) <= 1;
 }
 __device__ void enqueue_once(const FactArgs &A, int j) {
 	if (!(atomicOr(reinterpret_cast<unsigned *>(A.nstat) + j, ADM_QUEUED) & ADM_QUEUED)) q_push(A, j);
@@ -525,8 +526,9 @@ __device__ void admit_step(const FactArgs &A, int j, unsigned delta) {
 	const unsigned old = atomicSub(reinterpret_cast<unsigned *>(A.nstat) + j, delta);
 	const unsigned now = old - delta;
 	bool q = !admissible(old) && admissible(now);
-	if (delta == ADM_ONE_CLAIM && ((now >> 15) & 0x7fffu) == 0 && (now & 0x7fffu) == BSG_ADMIT_UNFINISHED + 1)
-		q = -q_backlog(A) > A.hold_max / 8 && *(volatile int *)A.nbig < BIG_SLOTS / 4;
+	const int unf = (int)(now & 0x7fffu);
+	if (!q && ((now >> 15) & 0x7fffu) == 0 && unf > 1 && unf <= 4)
+		q = -q_backlog(A) > (unf == 2 ? A.hold_max / 8 : A.hold_max) && *(volatile int *)A.nbig < BIG_SLOTS / 4;
 	if (q) enqueue_once(A, j);
 }
 
