@@ -506,7 +506,9 @@ __device__ __forceinline__ long long q_backlog(const FactArgs &A) {
 // row keeps one from the rows it waits for.  Never -> two -> up to four: IC2
 // 32^3 18.2 -> 12.2 -> 11.1 ms, with thresholds 1e-2 and 1e-4 30.7 (two) ->
 // 25.2, 80x72x65 66.7 -> 49.7 -> 49.7, block IC2 periodic 20^3 210 (two) -> 185,
-// 12^3 64 -> 48, ILU2 20^3 54 -> 42.5; up to eight: 174, 39 and 48.  (Always with
+// 12^3 64 -> 48, ILU2 20^3 54 -> 42.5.  Up to eight gives 171, 39 and 41, but
+// where all rows overflow they then go round the queue (4955 rows of 1500 members
+// 3.3 -> 5.0 s).  (Always with
 // two unfinished, waiting rows take the warps that others need: 80x72x65
 // 206 ms, 128^3 1.3 s.)  A row that another row waits for is queued earlier
 // (promoted) if nobody has queued it yet.  Bit 30 makes the first of these the
