@@ -91,7 +91,10 @@ __device__ __forceinline__ void devstat_fail(bsg_devstat *st, int code, int wher
 
 // Spin-wait bound: every device wait on another warp's result gives up after
 // this many nanoseconds of globaltimer time, reports BSG_ERR_TIMEOUT and
-// returns.  The default, two seconds, is far above any legitimate wait;
+// returns.  Where a wait may legitimately last as long as the call (a block of
+// an exact solve waiting for the blocks before it, a warp waiting for a row to
+// factor), the time counts from the last row that any warp finished.  The
+// default, two seconds, is far above any legitimate wait counted that way;
 // bsg_set_spin_limit_ns() changes it.  Every translation unit with waits
 // keeps its own copy in constant memory (static), set through
 // bsg_spin_limit_set_here() from that unit, for the current device.

@@ -11,7 +11,8 @@
 //   block of consecutive rows its CTA owns, and each lane waits on the entry it
 //   needs.  "Solved" is encoded in the value itself: y is pre-filled with a NaN
 //   bit pattern no arithmetic produces, and a 64-bit store publishes the result
-//   in one transaction.  Every wait is bounded by globaltimer (BSG_ERR_TIMEOUT).
+//   in one transaction.  A wait gives up (BSG_ERR_TIMEOUT) when globaltimer runs
+//   on for the limit without a row solved anywhere.
 // mode 1 -- Jacobi sweeps: y <- D^{-1}(x - N y) repeated nsweeps times from
 //   y = D^{-1} x; every sweep is a fully parallel pass over the factor (HBM
 //   bound: 4 B value (FP32) or 8 B (FP64) + 4 B column per entry).  It applies
@@ -75,24 +76,39 @@ __global__ void k_scale_vec(int n, const double *x, const double *d, double *y) 
 // 256 146 / 516, 512 152 / 566, 1024 158 / 634)
 #define TRSV_ROWS_MIN 256
 
+// The spin limit of a wait.  A block waits from the launch on for all the blocks
+// that come before it, so the limit counts from the last progress of the whole
+// solve: a warp adds to *solved after every 32 rows of its own and after its last,
+// and a wait that sees *solved move starts again.  (An add every eight rows, in the
+// row loop, costs 1.5 to 3 %.)
+struct TrsvLimit {
+	unsigned t0 = 0, seen = 0; // in units of 1024 ns (registers are short here)
+	// whether to give up: another warp failed, or the limit has passed
+	__device__ __forceinline__ bool over(const unsigned *solved, int row, bsg_devstat *st) {
+		if (*(volatile int *)&st->code != 0) return true;
+		const unsigned now = (unsigned)(globaltimer_ns() >> 10) | 1u, cnt = *(const volatile unsigned *)solved;
+		if (t0 == 0 || cnt != seen) {
+			t0 = now;
+			seen = cnt;
+		} else if (now - t0 > (unsigned)(BSG_SPIN_LIMIT_NS >> 10)) {
+			devstat_fail(st, BSG_ERR_TIMEOUT, row);
+			return true;
+		}
+		return false;
+	}
+};
+
 // The solved entry at p (shared or global), waiting for it; the spin limit or
 // another warp's failure gives 0.
-__device__ __forceinline__ unsigned long long trsv_wait(const double *p, int row, bsg_devstat *st) {
+__device__ __forceinline__ unsigned long long trsv_wait(const double *p, int row, const unsigned *solved,
+                                                        bsg_devstat *st) {
 	unsigned long long raw = ld_volatile_generic_u64(p);
 	if (raw != BSG_PENDING) return raw;
-	unsigned long long t0 = 0;
+	TrsvLimit limit;
 	for (unsigned it = 1;; it++) {
 		raw = ld_volatile_generic_u64(p);
 		if (raw != BSG_PENDING) return raw;
-		if ((it & 127) == 0) {
-			if (*(volatile int *)&st->code != 0) return 0;
-			const unsigned long long now = globaltimer_ns();
-			if (t0 == 0) t0 = now;
-			else if (now - t0 > BSG_SPIN_LIMIT_NS) {
-				devstat_fail(st, BSG_ERR_TIMEOUT, row);
-				return 0;
-			}
-		}
+		if ((it & 127) == 0 && limit.over(solved, row, st)) return 0;
 	}
 }
 
@@ -100,7 +116,7 @@ template <typename VT>
 __global__ void __launch_bounds__(TRSV_WARPS * 32, 1)
 k_trsv_blocks(int n, int lower, int block0, int rows, const int *__restrict__ perm, const int *__restrict__ rp,
               const int *__restrict__ ci, const VT *__restrict__ v, int skip_first, const double *__restrict__ dinv,
-              const double *__restrict__ x, double *y, bsg_devstat *st) {
+              const double *__restrict__ x, double *y, unsigned *solved, bsg_devstat *st) {
 	extern __shared__ double ys[]; // the block's solved rows, BSG_PENDING before
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int r0 = (block0 + blockIdx.x) * rows, cnt = min(rows, n - r0);
@@ -169,7 +185,7 @@ k_trsv_blocks(int n, int lower, int block0, int rows, const int *__restrict__ pe
 				const int tail = b + ((e - b - 1) / 32 - (TRSV_M - 1)) * 32;
 				for (int k = b + lane; k < tail; k += 32) {
 					const int col = ci[k];
-					s = fma((double)v[k], __longlong_as_double((long long)trsv_wait(entry(col), row, st)), s);
+					s = fma((double)v[k], __longlong_as_double((long long)trsv_wait(entry(col), row, solved, st)), s);
 				}
 				__syncwarp();
 			}
@@ -182,7 +198,7 @@ k_trsv_blocks(int n, int lower, int block0, int rows, const int *__restrict__ pe
 			}
 			// poll until at most one lane waits
 			unsigned wait;
-			unsigned long long t0 = 0;
+			TrsvLimit limit;
 			for (unsigned it = 1;; it++) {
 				bool mine = false;
 #pragma unroll
@@ -192,21 +208,12 @@ k_trsv_blocks(int n, int lower, int block0, int rows, const int *__restrict__ pe
 				}
 				wait = __ballot_sync(0xffffffffu, mine);
 				if ((wait & (wait - 1)) == 0) break;
-				if ((it & 127) == 0) { // the limit, or another warp's failure: leave the rest at 0
-					bool give = *(volatile int *)&st->code != 0;
-					const unsigned long long now = globaltimer_ns();
-					if (t0 == 0) t0 = now;
-					else if (!give && now - t0 > BSG_SPIN_LIMIT_NS) {
-						devstat_fail(st, BSG_ERR_TIMEOUT, row);
-						give = true;
-					}
-					if (__any_sync(0xffffffffu, give)) {
+				if ((it & 127) == 0 && __any_sync(0xffffffffu, limit.over(solved, row, st))) { // leave the rest at 0
 #pragma unroll
-						for (int u = 0; u < TRSV_M; u++)
-							if (raw[u] == BSG_PENDING) raw[u] = 0;
-						wait = 0;
-						break;
-					}
+					for (int u = 0; u < TRSV_M; u++)
+						if (raw[u] == BSG_PENDING) raw[u] = 0;
+					wait = 0;
+					break;
 				}
 			}
 			const int last = wait ? __ffs(wait) - 1 : 0; // the lane that finishes the row
@@ -230,7 +237,7 @@ k_trsv_blocks(int n, int lower, int block0, int rows, const int *__restrict__ pe
 #pragma unroll
 					for (int u = 0; u < TRSV_M; u++)
 						if (c[u] >= 0) {
-							if (raw[u] == BSG_PENDING) raw[u] = trsv_wait(src[u], row, st);
+							if (raw[u] == BSG_PENDING) raw[u] = trsv_wait(src[u], row, solved, st);
 							t = fma(a[u], __longlong_as_double((long long)raw[u]), t);
 						}
 				}
@@ -242,6 +249,7 @@ k_trsv_blocks(int n, int lower, int block0, int rows, const int *__restrict__ pe
 			}
 			__syncwarp();
 		}
+		if (lane == 0) atomicAdd(solved, 1u);
 		cur = nxt;
 	}
 }
@@ -469,12 +477,12 @@ int trisolve_impl(bsg_ctx *c, const bsg_fct *f, const TriOp &t, int mode, int ns
 				cudaFuncSetAttribute(k_trsv_blocks<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 				                     (int)sizeof(double) * TRSV_ROWS_MAX);
 				e = cudaLaunchKernelEx(&cfg, k_trsv_blocks<float>, n, t.lower, b0, rows, (const int *)f->d_perm, t.rp, t.ci,
-				                       t.vf, t.skip, t.dinv, x, y, c->d_stat);
+				                       t.vf, t.skip, t.dinv, x, y, c->d_counters + 1, c->d_stat);
 			} else {
 				cudaFuncSetAttribute(k_trsv_blocks<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 				                     (int)sizeof(double) * TRSV_ROWS_MAX);
 				e = cudaLaunchKernelEx(&cfg, k_trsv_blocks<double>, n, t.lower, b0, rows, (const int *)f->d_perm, t.rp, t.ci,
-				                       t.vd, t.skip, t.dinv, x, y, c->d_stat);
+				                       t.vd, t.skip, t.dinv, x, y, c->d_counters + 1, c->d_stat);
 			}
 			BSG_CUDA(e);
 		}

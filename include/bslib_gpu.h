@@ -104,7 +104,8 @@ int bsg_sync(bsg_ctx *ctx);
 /* Time limit of every device spin-wait (the sync-free triangular solves, the
  * factorisation scheduler, the tensor-core pipeline of the learned stage), in
  * nanoseconds of GPU time: a wait that reaches it gives up, the call returns
- * BSG_ERR_TIMEOUT and the context stays usable.  Default 2 s; accepted range
+ * BSG_ERR_TIMEOUT and the context stays usable.  Rows solved by other warps
+ * count as progress in an exact solve and start the time again.  Default 2 s; accepted range
  * 1 us .. 600 s.  It holds for the context's device, for every context on it,
  * from the next launch on; the call synchronises the context's stream first.
  * No counterpart in the reference (its loops have no waits). */
