@@ -59,9 +59,13 @@ __global__ void k_scale_vec(int n, const double *x, const double *d, double *y) 
 //    of warp_sum() would add to its own and adds them in that order, so the
 //    result has the bits of the plain reduction, without its shuffles after
 //    the wait.
-// All CTAs must be resident (a cooperative launch): the unsolved row that comes
-// first by (level, place in its list) depends on solved rows only, and its warp
-// has no earlier row left, so the solve always progresses.
+// Blocks are claimed from a counter in solve order (ascending for L, descending
+// for U).  A block's rows depend on rows of its own and of blocks claimed before,
+// whose CTAs run already or are done; within a block, the unsolved row that comes
+// first by (level, place in its list) waits for solved rows or other blocks only,
+// and its warp has no earlier row left.  So the solve always progresses, with any
+// number of CTAs resident: on a part of the GPU, beside other kernels, or with more
+// blocks than SMs.
 // Measured against one warp per row claimed in global level order with every
 // link through L2 (us per forward solve, before / after, FP64 IC2 tau 1e-3 of the
 // 7-point heat operator): 12^3 553 / 145, 32^3 1668 / 309, 47x40x33 3537 / 514,
@@ -114,12 +118,17 @@ __device__ __forceinline__ unsigned long long trsv_wait(const double *p, int row
 
 template <typename VT>
 __global__ void __launch_bounds__(TRSV_WARPS * 32, 1)
-k_trsv_blocks(int n, int lower, int block0, int rows, const int *__restrict__ perm, const int *__restrict__ rp,
+k_trsv_blocks(int n, int lower, int rows, const int *__restrict__ perm, const int *__restrict__ rp,
               const int *__restrict__ ci, const VT *__restrict__ v, int skip_first, const double *__restrict__ dinv,
-              const double *__restrict__ x, double *y, unsigned *solved, bsg_devstat *st) {
+              const double *__restrict__ x, double *y, unsigned *claim, unsigned *solved,
+              bsg_devstat *st) {
 	extern __shared__ double ys[]; // the block's solved rows, BSG_PENDING before
+	__shared__ unsigned block;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int r0 = (block0 + blockIdx.x) * rows, cnt = min(rows, n - r0);
+	if (threadIdx.x == 0) block = atomicAdd(claim, 1u);
+	for (int k = threadIdx.x; k < rows; k += blockDim.x) ys[k] = __longlong_as_double((long long)BSG_PENDING);
+	__syncthreads();
+	const int r0 = (int)(lower ? block : gridDim.x - 1 - block) * rows, cnt = min(rows, n - r0);
 	// item k of this warp: place warp + k TRSV_WARPS of the block's list (read backwards for U)
 	auto item = [&](int k) {
 		const int o = warp + k * TRSV_WARPS;
@@ -140,10 +149,8 @@ k_trsv_blocks(int n, int lower, int block0, int rows, const int *__restrict__ pe
 		return m;
 	};
 	int row1 = item(lane);
-	for (int k = threadIdx.x; k < cnt; k += blockDim.x) ys[k] = __longlong_as_double((long long)BSG_PENDING);
 	Meta cur = meta(row1);
 	row1 = item(32 + lane);
-	__syncthreads();
 	int nc[TRSV_M];
 	VT nv[TRSV_M];
 	auto load = [&](int b, int e) { // the last 32 TRSV_M entries of a row at most
@@ -290,8 +297,9 @@ __global__ void __launch_bounds__(256) k_trsv_jacobi(int n, const int *__restric
 	}
 }
 
-// y before an exact solve: nothing solved
-__global__ void k_fill_u64(long long n, unsigned long long *p, unsigned long long v) {
+// y before an exact solve: nothing solved, no block claimed
+__global__ void k_fill_u64(long long n, unsigned long long *p, unsigned long long v, unsigned *claim) {
+	if (blockIdx.x == 0 && threadIdx.x == 0) *claim = 0;
 	for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
 		p[i] = v;
 }
@@ -452,39 +460,21 @@ int trisolve_impl(bsg_ctx *c, const bsg_fct *f, const TriOp &t, int mode, int ns
 	const int n = f->n;
 	const bool use32 = f->fp32 != 0;
 	if (mode == 0) {
-		BSG_COUNT(1);
+		if (n == 0) return BSG_OK;
+		BSG_COUNT(2);
+		unsigned *claim = c->d_counters + 1, *solved = c->d_counters + 2;
 		const int fill = nb(n, 256) < BSG_SMS * 4 ? nb(n, 256) : BSG_SMS * 4;
-		k_fill_u64<<<fill, 256, 0, s>>>(n, (unsigned long long *)y, BSG_PENDING);
-		const int rows = f->trsv_rows, blocks = n > 0 ? (n + rows - 1) / rows : 0;
-		// at most one block per SM at a time: larger systems take several
-		// launches over consecutive blocks, in solve order
-		const int steps = (blocks + BSG_SMS - 1) / BSG_SMS;
-		for (int k = 0; k < steps; k++) {
-			const int b0 = (t.lower ? k : steps - 1 - k) * BSG_SMS;
-			cudaLaunchConfig_t cfg = {};
-			cfg.gridDim = dim3(blocks - b0 < BSG_SMS ? blocks - b0 : BSG_SMS);
-			cfg.blockDim = dim3(TRSV_WARPS * 32);
-			cfg.dynamicSmemBytes = sizeof(double) * rows;
-			cfg.stream = s;
-			cudaLaunchAttribute coop;
-			coop.id = cudaLaunchAttributeCooperative;
-			coop.val.cooperative = 1;
-			cfg.attrs = &coop;
-			cfg.numAttrs = 1;
-			BSG_COUNT(1);
-			cudaError_t e;
-			if (use32) {
-				cudaFuncSetAttribute(k_trsv_blocks<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-				                     (int)sizeof(double) * TRSV_ROWS_MAX);
-				e = cudaLaunchKernelEx(&cfg, k_trsv_blocks<float>, n, t.lower, b0, rows, (const int *)f->d_perm, t.rp, t.ci,
-				                       t.vf, t.skip, t.dinv, x, y, c->d_counters + 1, c->d_stat);
-			} else {
-				cudaFuncSetAttribute(k_trsv_blocks<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-				                     (int)sizeof(double) * TRSV_ROWS_MAX);
-				e = cudaLaunchKernelEx(&cfg, k_trsv_blocks<double>, n, t.lower, b0, rows, (const int *)f->d_perm, t.rp, t.ci,
-				                       t.vd, t.skip, t.dinv, x, y, c->d_counters + 1, c->d_stat);
-			}
-			BSG_CUDA(e);
+		k_fill_u64<<<fill, 256, 0, s>>>(n, (unsigned long long *)y, BSG_PENDING, claim);
+		const int rows = f->trsv_rows, blocks = (n + rows - 1) / rows;
+		const int smem = (int)sizeof(double) * rows, most = (int)sizeof(double) * TRSV_ROWS_MAX;
+		if (use32) {
+			BSG_CUDA(cudaFuncSetAttribute(k_trsv_blocks<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+			k_trsv_blocks<float><<<blocks, TRSV_WARPS * 32, smem, s>>>(n, t.lower, rows, f->d_perm, t.rp, t.ci, t.vf, t.skip,
+			                                                           t.dinv, x, y, claim, solved, c->d_stat);
+		} else {
+			BSG_CUDA(cudaFuncSetAttribute(k_trsv_blocks<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+			k_trsv_blocks<double><<<blocks, TRSV_WARPS * 32, smem, s>>>(n, t.lower, rows, f->d_perm, t.rp, t.ci, t.vd, t.skip,
+			                                                            t.dinv, x, y, claim, solved, c->d_stat);
 		}
 		return cudaGetLastError() == cudaSuccess ? BSG_OK : BSG_ERR_CUDA;
 	}
