@@ -70,8 +70,8 @@ __global__ void k_scale_vec(int n, const double *x, const double *d, double *y) 
 // link through L2 (us per forward solve, before / after, FP64 IC2 tau 1e-3 of the
 // 7-point heat operator): 12^3 553 / 145, 32^3 1668 / 309, 47x40x33 3537 / 514,
 // 128^3 18690 / 5470; IC(0) 128^3 2075 / 1170; 2-D 500^2 22752 / 1836; a chain of
-// 100000 rows 437 / 21 ms (0.21 us a link).  A random graph with 30 levels has
-// no links to keep inside a block: 249 / 285.
+// 100000 rows 437 / 21 ms (0.21 us a link).  Factors without locality go by rows
+// as before (k_trsv_rows, see trsv_scattered).
 #define TRSV_WARPS 32 // 24 warps: 47x40x33 580, 128^3 5520; 16: 760, 6600
 #define TRSV_M 2 // entries of a row each lane holds (32 TRSV_M a row; longer rows walk their head first)
 #define TRSV_ROWS_MAX 28000 // rows of a block: 8 bytes each in shared memory
@@ -261,18 +261,79 @@ k_trsv_blocks(int n, int lower, int rows, const int *__restrict__ perm, const in
 	}
 }
 
-// Sort keys of the solve order: the row's block, then its level; *most gets the
-// largest level.
+// The exact solve where blocks do not pay (see trsv_scattered): a warp per row, the
+// rows claimed in global level order (perm, read backwards for U), so that the
+// rows in flight are those of the current wavefront, wherever they lie.  Bound: a
+// link through L2, about 4 us a level, and the claims, 0.7 ns a row.
+template <typename VT>
+__global__ void __launch_bounds__(256) k_trsv_rows(int n, int lower, const int *__restrict__ perm,
+                                                   const int *__restrict__ rp, const int *__restrict__ ci,
+                                                   const VT *__restrict__ v, int skip_first,
+                                                   const double *__restrict__ dinv, const double *__restrict__ x,
+                                                   double *y, unsigned *claim, bsg_devstat *st) {
+	const int lane = threadIdx.x & 31;
+	for (;;) {
+		int t = 0;
+		if (lane == 0) t = (int)atomicAdd(claim, 1u);
+		t = __shfl_sync(0xffffffffu, t, 0);
+		if (t >= n) return;
+		const int row = perm[lower ? t : n - 1 - t];
+		const int b = rp[row] + skip_first, e = rp[row + 1];
+		double s = 0.0;
+		for (int k = b + lane; k < e; k += 32) {
+			const int c = ci[k];
+			unsigned long long raw = ld_volatile_u64(y + c);
+			if (raw == BSG_PENDING) {
+				TrsvLimit limit; // (claims are progress)
+				for (unsigned it = 1;; it++) {
+					__nanosleep(32);
+					raw = ld_volatile_u64(y + c);
+					if (raw != BSG_PENDING) break;
+					if ((it & 127) == 0 && limit.over(claim, row, st)) {
+						raw = 0;
+						break;
+					}
+				}
+			}
+			s = fma((double)v[k], __longlong_as_double((long long)raw), s);
+		}
+		s = warp_sum(s);
+		if (lane == 0) st_volatile_f64(y + row, (x[row] - s) * dinv[row]);
+	}
+}
+
+// Sort keys of the solve order: the row's block (all in one for rows == 0), then
+// its level; *most gets the largest level.
 __global__ void k_trsv_keys(int n, int rows, const int *lev, unsigned long long *keys, int *vals) {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
-	keys[i] = ((unsigned long long)(unsigned)(i / rows) << 32) | (unsigned)lev[i];
+	keys[i] = ((unsigned long long)(unsigned)(rows ? i / rows : 0) << 32) | (unsigned)lev[i];
 	vals[i] = i;
 }
 __global__ void k_trsv_levels(int n, const int *lev, int *most) {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	const int m = __reduce_max_sync(0xffffffffu, i < n ? lev[i] : 0);
 	if ((threadIdx.x & 31) == 0) atomicMax(most, m);
+}
+// most[l] = the most rows of level l in one block (sorted keys: a run per block
+// and level)
+__global__ void k_trsv_crowd(int n, const unsigned long long *keys, int *most) {
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= n) return;
+	const unsigned long long k = keys[i];
+	if (i > 0 && keys[i - 1] == k) return;
+	int lo = i + 1, hi = n; // the first place with another key
+	while (lo < hi) {
+		const int mid = lo + (hi - lo) / 2;
+		if (keys[mid] == k) lo = mid + 1;
+		else hi = mid;
+	}
+	atomicMax(most + (unsigned)k, lo - i);
+}
+__global__ void k_trsv_sum(int n, const int *v, int *sum) {
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	const int t = __reduce_add_sync(0xffffffffu, i < n ? v[i] : 0);
+	if ((threadIdx.x & 31) == 0 && t) atomicAdd(sum, t);
 }
 
 template <int G, typename VT>
@@ -329,9 +390,27 @@ inline int nb(long long n, int t) { return n > 0 ? (int)((n + t - 1) / t) : 1; }
 int bsg_strict_transpose(bsg_ctx *c, int n, const int *ia, const int *ja, int nnz, int **it_o, int **jt_o,
                          int **perm_o, int *nnz_o);
 
+// Whether an exact solve goes by rows in global level order instead of by blocks:
+// crowd is the sum over the levels of the most rows of the level in one block.  The
+// block with the most rows of a level holds the level up, 32 rows a microsecond;
+// without blocks a level takes 4 us and a row 0.7 ns.  So wavefronts that stand in
+// few blocks (windowed graphs) or wide ones without locality (permuted grids) go by
+// rows.  Below 50000 rows blocks were never slower.  us a solve, by rows / by blocks,
+// * the one taken: IC(0) of random graphs with 3 neighbours within +-w: 300000 rows,
+// w 1000 8940 / 6960*, 3000 3095* / 4650, 30000 243* / 655, any 235 / 214*; 1000000
+// rows, w 30000 760* / 6030, any 692 / 657*; 8 neighbours, 300000 rows, w 3000 7660 /
+// 7390*, 100000 239* / 556; permuted 64^3 grid, IC2 273* / 439, IC(0) 208 / 192*;
+// natural 128^3, IC(0) 2070 / 1160*.
+#define TRSV_SCATTER_MIN 50000
+static bool trsv_scattered(int n, int levels, double crowd) {
+	const double blocks = 20.0 + 0.9 * crowd / TRSV_WARPS, rows1 = 4.0 * levels - 15.0, rows2 = 25.0 + 0.69e-3 * n;
+	return blocks > (rows1 > rows2 ? rows1 : rows2);
+}
+
 // The exact solves' order of f's n rows from their levels (ascending depth in
 // the forward solve's dependency graph): blocks of f->trsv_rows consecutive
-// rows, by (level, index) inside a block, in f->d_perm; sets levels_l / levels_u.
+// rows, by (level, index) inside a block, in f->d_perm; or, with trsv_rows 0, all
+// rows by (level, index).  Sets levels_l / levels_u.
 int bsg_trsv_schedule(bsg_ctx *c, bsg_fct *f, const int *lev) {
 	cudaStream_t s = c->stream;
 	const int n = f->n;
@@ -351,24 +430,40 @@ int bsg_trsv_schedule(bsg_ctx *c, bsg_fct *f, const int *lev) {
 	int bits = 32;
 	while ((1ll << (bits - 32)) < (n + rows - 1) / rows) bits++;
 	unsigned long long *keys = nullptr, *k2 = nullptr;
-	int *vals = nullptr, *most = nullptr, top = 0;
+	int *vals = nullptr, *most = nullptr, *crowd = nullptr, top[2] = {0, 0}; // largest level, sum of crowd
 	void *tmp = nullptr;
 	size_t tb = 0;
 	BSG_CUDA(cudaMallocAsync(&keys, sizeof(unsigned long long) * n, s));
 	BSG_CUDA(cudaMallocAsync(&k2, sizeof(unsigned long long) * n, s));
 	BSG_CUDA(cudaMallocAsync(&vals, sizeof(int) * n, s));
-	BSG_CUDA(cudaMallocAsync(&most, sizeof(int), s));
-	BSG_CUDA(cudaMemsetAsync(most, 0, sizeof(int), s));
+	BSG_CUDA(cudaMallocAsync(&most, sizeof(top), s));
+	BSG_CUDA(cudaMemsetAsync(most, 0, sizeof(top), s));
 	BSG_COUNT(2);
 	k_trsv_levels<<<nb(n, 256), 256, 0, s>>>(n, lev, most);
 	k_trsv_keys<<<nb(n, 256), 256, 0, s>>>(n, f->trsv_rows, lev, keys, vals);
 	BSG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
 	BSG_CUDA(cudaMallocAsync(&tmp, tb > 0 ? tb : 1, s));
 	BSG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
-	BSG_CUDA(cudaMemcpyAsync(&top, most, sizeof(int), cudaMemcpyDeviceToHost, s));
+	if (n >= TRSV_SCATTER_MIN) {
+		BSG_CUDA(cudaMallocAsync(&crowd, sizeof(int) * n, s)); // (levels < n)
+		BSG_CUDA(cudaMemsetAsync(crowd, 0, sizeof(int) * n, s));
+		BSG_COUNT(2);
+		k_trsv_crowd<<<nb(n, 256), 256, 0, s>>>(n, k2, crowd);
+		k_trsv_sum<<<nb(n, 256), 256, 0, s>>>(n, crowd, most + 1);
+	}
+	BSG_CUDA(cudaMemcpyAsync(top, most, sizeof(top), cudaMemcpyDeviceToHost, s));
 	BSG_CUDA(cudaStreamSynchronize(s));
-	f->levels_l = f->levels_u = top + 1;
-	for (void *q : {(void *)keys, (void *)k2, (void *)vals, (void *)most, tmp}) cudaFreeAsync(q, s);
+	f->levels_l = f->levels_u = top[0] + 1;
+	// more blocks than SMs run in turn
+	const long long turns = ((n + rows - 1) / rows + BSG_SMS - 1) / BSG_SMS;
+	if (n >= TRSV_SCATTER_MIN && trsv_scattered(n, f->levels_l, (double)top[1] * turns)) {
+		f->trsv_rows = 0;
+		BSG_COUNT(1);
+		k_trsv_keys<<<nb(n, 256), 256, 0, s>>>(n, 0, lev, keys, vals);
+		BSG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
+	}
+	for (void *q : {(void *)keys, (void *)k2, (void *)vals, (void *)most, (void *)crowd, tmp})
+		if (q) cudaFreeAsync(q, s);
 	return BSG_OK;
 }
 
@@ -465,7 +560,18 @@ int trisolve_impl(bsg_ctx *c, const bsg_fct *f, const TriOp &t, int mode, int ns
 		unsigned *claim = c->d_counters + 1, *solved = c->d_counters + 2;
 		const int fill = nb(n, 256) < BSG_SMS * 4 ? nb(n, 256) : BSG_SMS * 4;
 		k_fill_u64<<<fill, 256, 0, s>>>(n, (unsigned long long *)y, BSG_PENDING, claim);
-		const int rows = f->trsv_rows, blocks = (n + rows - 1) / rows;
+		const int rows = f->trsv_rows;
+		if (!rows) {
+			const int grid = (n + 7) / 8 < BSG_SMS * 8 ? (n + 7) / 8 : BSG_SMS * 8;
+			if (use32)
+				k_trsv_rows<float><<<grid, 256, 0, s>>>(n, t.lower, f->d_perm, t.rp, t.ci, t.vf, t.skip, t.dinv, x, y, claim,
+				                                       c->d_stat);
+			else
+				k_trsv_rows<double><<<grid, 256, 0, s>>>(n, t.lower, f->d_perm, t.rp, t.ci, t.vd, t.skip, t.dinv, x, y, claim,
+				                                        c->d_stat);
+			return cudaGetLastError() == cudaSuccess ? BSG_OK : BSG_ERR_CUDA;
+		}
+		const int blocks = (n + rows - 1) / rows;
 		const int smem = (int)sizeof(double) * rows, most = (int)sizeof(double) * TRSV_ROWS_MAX;
 		if (use32) {
 			BSG_CUDA(cudaFuncSetAttribute(k_trsv_blocks<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
