@@ -1566,6 +1566,7 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 		}
 		res = __shfl_sync(0xffffffffu, res, 0);
 		rec = __shfl_sync(0xffffffffu, rec, 0);
+		__syncwarp(); // lane 0's acquire covers the other lanes' loads of that row (a shuffle orders no memory)
 		tail0 = clock64();
 		waited = true;
 		pc.v[FS_CYC_BLOCKED] += tail0 - k2;
