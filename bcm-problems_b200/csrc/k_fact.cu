@@ -146,7 +146,7 @@ struct FactArgs {
 	int *big_owner;            // 1 while a warp holds that workspace
 	int *nhold;                // warps holding their row for a member nobody computes
 	int *nbig;                 // workspaces taken
-	int *novf;                 // rows that took one so far, without those of A's longest rows
+	int *novf;                 // rows that took one so far, each once, without those that A itself makes long
 	int hold_max;              // at most this many (half the warps)
 };
 
@@ -1764,9 +1764,13 @@ __global__ void __launch_bounds__(fact_warps<BLK, WIDE> * 32, FACT_MINB) k_fact_
 				}
 				if (slot >= 0) {
 					atomicAdd(A.nbig, 1);
-					// (rows that A itself makes long are left out: the
-					// wide kernel need not take them either)
-					if (!BLK && !WIDE && A.iu[i + 1] - A.iu[i] < HCAP) {
+					// (rows that A itself makes long, by their own entries
+					// or by their neighbours before them, are left out: the
+					// wide kernel need not take them either.  lev[i], set
+					// when the row is finished, marks those counted: a row
+					// that parks comes here again)
+					if (!BLK && !WIDE && A.iu[i + 1] - A.iu[i] < s.hcap && A.it[i + 1] - A.it[i] <= s.cmax &&
+					    atomicExch(A.lev + i, -1) == 0) {
 						const int novf = atomicAdd(A.novf, 1) + 1, done = *(volatile int *)A.done_count;
 						if (novf > WIDE_MIN + done / WIDE_DIV && done < A.n / 2)
 							devstat_fail(A.st, BSG_ERR_WORKSPACE, i, SITE_WIDE);
