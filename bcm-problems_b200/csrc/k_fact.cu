@@ -1566,7 +1566,6 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 		}
 		res = __shfl_sync(0xffffffffu, res, 0);
 		rec = __shfl_sync(0xffffffffu, rec, 0);
-		__syncwarp(); // lane 0's acquire covers the other lanes' loads of that row (a shuffle orders no memory)
 		tail0 = clock64();
 		waited = true;
 		pc.v[FS_CYC_BLOCKED] += tail0 - k2;
@@ -1577,6 +1576,7 @@ __device__ int try_row(const FactArgs &A, WS &s, int i, int lane, PhaseClock &pc
 		}
 		pass = true;
 		if constexpr (alone) {
+			__syncwarp(); // lane 0's acquire covers the other lanes' loads of that row (a shuffle orders no memory)
 			if (lane == 0) accraw = __ldcg(A.acc + i); // complete if this was the last member
 			if (take_member(A, s, i, tw, rec, lane, levmax, nopen, ncol, err)) {
 				pc.v[FS_CLOSED]++;
