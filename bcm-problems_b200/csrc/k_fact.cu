@@ -98,14 +98,21 @@
 #ifndef WSETCAP
 #define WSETCAP 128 // far members (hash slots, a power of two)
 #endif
-// block rows (3 x 3 blocks): mask columns and members of the shared
-// workspace, member bitmap window.  512 of each leave room for one CTA of two
-// warps on an SM and still pay, since rows in global memory hold up all others
-// (256 of each -> 512: periodic IC2 of 20^3 block rows 326 -> 206 ms, 12^3
-// 104 -> 64, clamped 44^3 150 -> 134, ILU2 20^3 64 -> 54, 36^3 125 -> 110).
-// 1024 columns, or three warps, give no more.
-#define HCAP_BLK 512
-#define CMAX_BLK 512
+// Block rows (3 x 3 blocks): mask columns and members of the shared workspace,
+// member bitmap window.  256 of each let six warps (IC2) or four (ILU2) stand on an
+// SM; the wide form, 512 of each, two, which pays where rows overflow, since rows
+// in global memory hold up all others (ms, narrow / wide: periodic IC2 of 12^3 block
+// rows at 1e-3 56 / 44, clamped 20^3 at 3e-4 451 / 129), and costs where they fit
+// and the front is broad (clamped, 1e-2, 36^3 77 / 90, 48^3 20 / 27, 64^3 35 / 105,
+// 72^3 44 / 162).  So up to BLK_WIDE_ROWS rows, where few warps find work, the
+// factor takes the wide form at once (28^3 at 1e-3: narrow 56, wide 60; at 3e-4,
+// where the narrow one gives up, 241 / 225), larger ones start with the narrow
+// one and its rule for giving up.  1024 columns, or three warps, give no more.
+#define HCAP_BLK 256
+#define CMAX_BLK 256
+#define HCAP_BLK_WIDE 512
+#define CMAX_BLK_WIDE 512
+#define BLK_WIDE_ROWS 32768
 #define MWIN_BLK 8192
 #define FACT_WARPS_BLK 2 // warps of a CTA in block mode (larger workspaces)
 #define W_EMPTY (-1)
@@ -171,8 +178,8 @@ struct PhaseClock {
 template <bool ILU, bool BLK = false, bool WIDE = false>
 struct SmemWS {
 	static constexpr bool big = false, ilu = ILU, blk = BLK;
-	static constexpr int cmax = BLK ? CMAX_BLK : WIDE ? CMAX_WIDE : CMAX,
-	                     hcap = BLK ? HCAP_BLK : WIDE ? HCAP_WIDE : HCAP, pfcap = PFCAP, wcap = WSETCAP,
+	static constexpr int cmax = BLK ? (WIDE ? CMAX_BLK_WIDE : CMAX_BLK) : WIDE ? CMAX_WIDE : CMAX,
+	                     hcap = BLK ? (WIDE ? HCAP_BLK_WIDE : HCAP_BLK) : WIDE ? HCAP_WIDE : HCAP, pfcap = PFCAP, wcap = WSETCAP,
 	                     mwin = BLK ? MWIN_BLK : MWIN;
 	int W[cmax];           // members (discovery order, then sorted)
 	int Wp[cmax];          // pool index of column i in that row (stored members)
@@ -1769,7 +1776,7 @@ __global__ void __launch_bounds__(fact_warps<BLK, WIDE> * 32, FACT_MINB) k_fact_
 					// wide kernel need not take them either.  lev[i], set
 					// when the row is finished, marks those counted: a row
 					// that parks comes here again)
-					if (!BLK && !WIDE && A.iu[i + 1] - A.iu[i] < s.hcap && A.it[i + 1] - A.it[i] <= s.cmax &&
+					if (!WIDE && A.iu[i + 1] - A.iu[i] < s.hcap && A.it[i + 1] - A.it[i] <= s.cmax &&
 					    atomicExch(A.lev + i, -1) == 0) {
 						const int novf = atomicAdd(A.novf, 1) + 1, done = *(volatile int *)A.done_count;
 						if (novf > WIDE_MIN + done / WIDE_DIV && done < A.n / 2)
@@ -2179,17 +2186,8 @@ int bsg_bfact_dyn(bsg_ctx *c, int nb, int sym, const bsg_param *p, const int *bi
 	BSG_CUDA(cudaMallocAsync(&pool_len, sizeof(unsigned long long), st));
 	BSG_CUDA(cudaMallocAsync(&qhead, sizeof(unsigned long long), st));
 	BSG_CUDA(cudaMallocAsync(&qtail, sizeof(unsigned long long), st));
-	void (*kern)(FactArgs) = kind == 1 ? k_fact_rows<true, true, false> : k_fact_rows<false, true, false>;
-	const size_t smem = (kind == 1 ? sizeof(SmemWS<true, true>) : sizeof(SmemWS<false, true>)) * FACT_WARPS_BLK;
 	const size_t big = kind == 1 ? GlobWS<true, true>::bytes : GlobWS<false, true>::bytes;
-	BSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-	int per_sm = 0;
-	BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FACT_WARPS_BLK * 32, smem));
-	if (per_sm < 1) per_sm = 1;
-	int grid = per_sm * BSG_SMS;
-	const int need = (nb + FACT_WARPS_BLK - 1) / FACT_WARPS_BLK;
-	if (grid > need) grid = need;
-	if (grid < 1) grid = 1;
+	int grid = 1;
 	FactArgs A;
 	A.n = nb; A.kind = kind;
 	A.iu = bia; A.ju = bja; A.al = bal; A.au = bau;
@@ -2207,13 +2205,13 @@ int bsg_bfact_dyn(bsg_ctx *c, int nb, int sym, const bsg_param *p, const int *bi
 	BSG_CUDA(cudaMallocAsync(&A.big_owner, sizeof(int) * (BIG_SLOTS + 3), st));
 	A.nhold = A.big_owner + BIG_SLOTS;
 	A.nbig = A.nhold + 1;
-	A.novf = A.nbig + 1; // (not counted for block rows)
-	A.hold_max = grid * FACT_WARPS_BLK / 2;
+	A.novf = A.nbig + 1;
 	BSG_CUDA(cudaMallocAsync(&A.stats, sizeof(unsigned long long) * FACT_NSTAT, st));
 	// The pool first holds 8 blocks per block of A (block IC2 / ILU2 keep
 	// about 4); a factor that needs more is computed again with the pool
 	// the memory parameter allows.
-	for (double memu = mem < 8.0 ? mem : 8.0;; memu = mem) {
+	double memu = mem < 8.0 ? mem : 8.0;
+	for (bool wide = nb <= BLK_WIDE_ROWS;;) {
 		long long cap = (long long)(memu * (double)nnzb) + 8LL * nb + 1024;
 		if (cap > 0x7ffffff0LL) cap = 0x7ffffff0LL;
 		if (cudaMallocAsync(&cf, sizeof(unsigned) * cap, st) != cudaSuccess ||
@@ -2233,19 +2231,33 @@ int bsg_bfact_dyn(bsg_ctx *c, int nb, int sym, const bsg_param *p, const int *bi
 		BSG_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * 3 * (size_t)nb, st));
 		k_fill_int<<<BSG_SMS * 4, 256, 0, st>>>(qcap, queue, -1);
 		k_fact_seed<<<nb_blocks(nb), 256, 0, st>>>(A);
+		void (*kern)(FactArgs) = kind == 1 ? (wide ? k_fact_rows<true, true, true> : k_fact_rows<true, true, false>)
+		                                   : (wide ? k_fact_rows<false, true, true> : k_fact_rows<false, true, false>);
+		const size_t ws = kind == 1 ? (wide ? sizeof(SmemWS<true, true, true>) : sizeof(SmemWS<true, true>))
+		                            : (wide ? sizeof(SmemWS<false, true, true>) : sizeof(SmemWS<false, true>));
+		const size_t smem = ws * FACT_WARPS_BLK;
+		BSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		int per_sm = 0;
+		BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FACT_WARPS_BLK * 32, smem));
+		grid = (per_sm < 1 ? 1 : per_sm) * BSG_SMS;
+		const int need = (nb + FACT_WARPS_BLK - 1) / FACT_WARPS_BLK;
+		if (grid > need) grid = need;
+		if (grid < 1) grid = 1;
+		A.hold_max = grid * FACT_WARPS_BLK / 2;
 		kern<<<grid, FACT_WARPS_BLK * 32, smem, st>>>(A);
 		BSG_CUDA(cudaGetLastError());
 		bsg_devstat h;
 		BSG_CUDA(cudaMemcpyAsync(&h, c->d_stat, sizeof(h), cudaMemcpyDeviceToHost, st));
 		BSG_CUDA(cudaStreamSynchronize(st));
-		if (h.code == BSG_ERR_WORKSPACE && h.pad[0] == 6 && memu < mem) { // the pool was too small
-			cudaFreeAsync(cf, st);
-			cudaFreeAsync(pl, st);
-			if (pu) cudaFreeAsync(pu, st);
-			cf = nullptr; pl = pu = nullptr;
-			continue;
-		}
-		break;
+		const bool more = h.code == BSG_ERR_WORKSPACE && h.pad[0] == 6 && memu < mem; // the pool was too small
+		const bool widen = h.code == BSG_ERR_WORKSPACE && h.pad[0] == SITE_WIDE;
+		if (!more && !widen) break;
+		cudaFreeAsync(cf, st);
+		cudaFreeAsync(pl, st);
+		if (pu) cudaFreeAsync(pu, st);
+		cf = nullptr; pl = pu = nullptr;
+		if (more) memu = mem;
+		else wide = true;
 	}
 	rc = bsg_check_devstat(c);
 	cudaMemcpyAsync(g_fact_stats, A.stats, sizeof(g_fact_stats), cudaMemcpyDeviceToHost, st);
