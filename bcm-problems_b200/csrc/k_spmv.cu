@@ -218,11 +218,19 @@ __global__ void __launch_bounds__(256, 4) k_spmv_bsr3_il(int nb, int nr, const i
 	}
 }
 
-// Whether products of five or six vectors go interleaved: enough rows to pay for
-// the interleaving, and no capture going on (the workspace comes from the
-// stream's pool).
+// Whether products of five or six vectors go interleaved: enough blocks to pay for
+// the interleaving, which takes a launch and a pass over the vectors, or vectors of
+// more than L2 holds, and no capture going on (the workspace comes from the
+// stream's pool).  us for six and for 11 vectors, strided / interleaved, * the one
+// taken: 6000 block rows, 4 blocks each 7.5* / 10.5 and 14.6* / 20.8, 16 blocks
+// 12.6* / 12.5 and 22.7* / 24.8, 27 blocks 20.5 / 12.6* and 33.1 / 24.9*; 20000
+// rows, 8 blocks 20.7* / 18.6 and 35.1* / 36.9, 10 blocks 31.5 / 22.1* and 51.5 /
+// 43.1*; 60000 rows, 4 blocks 37* / 36 and 68* / 72, 8 blocks 52 / 38* and 89 /
+// 76*; 300000 rows, 1 block 135* / 135 and 277* / 267, 6 blocks 231 / 148* and 361 /
+// 293*; 400000 rows, 1 block 228 / 179* and 381 / 354*.
 bool bsr3_il_applies(const bsg_mat *m, cudaStream_t s) {
 	if (m->n < 6000) return false;
+	if (m->n < 400000 && (long long)m->nnz < 5LL * m->n + 100000) return false;
 	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
 	if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
 		cudaGetLastError();
