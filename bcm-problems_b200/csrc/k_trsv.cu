@@ -429,23 +429,31 @@ int bsg_trsv_schedule(bsg_ctx *c, bsg_fct *f, const int *lev) {
 	f->trsv_rows = (int)rows;
 	int bits = 32;
 	while ((1ll << (bits - 32)) < (n + rows - 1) / rows) bits++;
-	unsigned long long *keys = nullptr, *k2 = nullptr;
-	int *vals = nullptr, *most = nullptr, *crowd = nullptr, top[2] = {0, 0}; // largest level, sum of crowd
-	void *tmp = nullptr;
+	struct Tmp { // freed on every way out
+		cudaStream_t s;
+		void *p = nullptr;
+		~Tmp() {
+			if (p) cudaFreeAsync(p, s);
+		}
+	} dkeys{s}, dk2{s}, dvals{s}, dmost{s}, dcrowd{s}, dtmp{s};
+	int top[2] = {0, 0}; // largest level, sum of crowd
 	size_t tb = 0;
-	BSG_CUDA(cudaMallocAsync(&keys, sizeof(unsigned long long) * n, s));
-	BSG_CUDA(cudaMallocAsync(&k2, sizeof(unsigned long long) * n, s));
-	BSG_CUDA(cudaMallocAsync(&vals, sizeof(int) * n, s));
-	BSG_CUDA(cudaMallocAsync(&most, sizeof(top), s));
+	BSG_CUDA(cudaMallocAsync(&dkeys.p, sizeof(unsigned long long) * n, s));
+	BSG_CUDA(cudaMallocAsync(&dk2.p, sizeof(unsigned long long) * n, s));
+	BSG_CUDA(cudaMallocAsync(&dvals.p, sizeof(int) * n, s));
+	BSG_CUDA(cudaMallocAsync(&dmost.p, sizeof(top), s));
+	unsigned long long *keys = (unsigned long long *)dkeys.p, *k2 = (unsigned long long *)dk2.p;
+	int *vals = (int *)dvals.p, *most = (int *)dmost.p;
 	BSG_CUDA(cudaMemsetAsync(most, 0, sizeof(top), s));
 	BSG_COUNT(2);
 	k_trsv_levels<<<nb(n, 256), 256, 0, s>>>(n, lev, most);
 	k_trsv_keys<<<nb(n, 256), 256, 0, s>>>(n, f->trsv_rows, lev, keys, vals);
 	BSG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
-	BSG_CUDA(cudaMallocAsync(&tmp, tb > 0 ? tb : 1, s));
-	BSG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
+	BSG_CUDA(cudaMallocAsync(&dtmp.p, tb > 0 ? tb : 1, s));
+	BSG_CUDA(cub::DeviceRadixSort::SortPairs(dtmp.p, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
 	if (n >= TRSV_SCATTER_MIN) {
-		BSG_CUDA(cudaMallocAsync(&crowd, sizeof(int) * n, s)); // (levels < n)
+		BSG_CUDA(cudaMallocAsync(&dcrowd.p, sizeof(int) * n, s)); // (levels < n)
+		int *crowd = (int *)dcrowd.p;
 		BSG_CUDA(cudaMemsetAsync(crowd, 0, sizeof(int) * n, s));
 		BSG_COUNT(2);
 		k_trsv_crowd<<<nb(n, 256), 256, 0, s>>>(n, k2, crowd);
@@ -460,10 +468,8 @@ int bsg_trsv_schedule(bsg_ctx *c, bsg_fct *f, const int *lev) {
 		f->trsv_rows = 0;
 		BSG_COUNT(1);
 		k_trsv_keys<<<nb(n, 256), 256, 0, s>>>(n, 0, lev, keys, vals);
-		BSG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
+		BSG_CUDA(cub::DeviceRadixSort::SortPairs(dtmp.p, tb, keys, k2, vals, f->d_perm, n, 0, bits, s));
 	}
-	for (void *q : {(void *)keys, (void *)k2, (void *)vals, (void *)most, (void *)crowd, tmp})
-		if (q) cudaFreeAsync(q, s);
 	return BSG_OK;
 }
 
