@@ -243,7 +243,7 @@ struct bsg_fct {
 	float *d_ur_f, *d_lr_f;       // FP32 strict values
 	int nnz_strict;
 	int *d_perm;                  // exact solves: rows by (block, forward-solve level, index)
-	int trsv_rows;                // consecutive rows a block
+	int trsv_rows;                // consecutive rows a block; 0: one block of all, solved row by row
 	bsg_sell sl, su;              // SELL-32 strict L / U rows (Jacobi sweeps), FP64 or FP32
 	int levels_l, levels_u;       // dependency depth
 	double density, density2;

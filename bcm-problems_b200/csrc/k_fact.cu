@@ -73,7 +73,7 @@
 // rows overflow takes them (k_fact_rows<.., WIDE>): the kernel gives up, in
 // the first half of the rows, once more than WIDE_MIN + done / WIDE_DIV rows
 // did, and the factor starts again with the wide one (IC2, tau 2e-4, 24^3:
-// 293 -> 89 ms; a divisor of 16 gives 95, of 8 118, of 4 150; no factor whose
+// 293 ms without, 88 with; a divisor of 16 gives 95, of 8 118, of 4 150; no factor whose
 // rows fit takes the wide kernel).  The factor does not depend on the
 // schedule, so both give the same bits.
 #define CMAX 192   // members of C(i)
@@ -84,6 +84,7 @@
 #define FACT_WARPS_WIDE 2
 #define WIDE_MIN 64
 #define WIDE_DIV 32
+#define SITE_WIDE 9 // BSG_ERR_WORKSPACE there: the factor wants the wide kernel
 // capacities of the global-memory workspaces that take the rows that do not
 // fit the shared one (about 0.7 MB each), and how many there are
 #define BIG_SLOTS 64
@@ -102,7 +103,7 @@
 // member bitmap window.  256 of each let six warps (IC2) or four (ILU2) stand on an
 // SM; the wide form, 512 of each, two, which pays where rows overflow, since rows
 // in global memory hold up all others (ms, narrow / wide: periodic IC2 of 12^3 block
-// rows at 1e-3 56 / 44, clamped 20^3 at 3e-4 451 / 129), and costs where they fit
+// rows at 1e-3 56 / 44, periodic 8^3 14.7 / 11.6), and costs where they fit
 // and the front is broad (clamped, 1e-2, 36^3 77 / 90, 48^3 20 / 27, 64^3 35 / 105,
 // 72^3 44 / 162).  So up to BLK_WIDE_ROWS rows, where few warps find work, the
 // factor takes the wide form at once (28^3 at 1e-3: narrow 56, wide 60; at 3e-4,
@@ -119,7 +120,6 @@
 #define W_CLOSED (-2)
 
 // row record: bit 63 done | bits 32..62 pool offset | bits 0..15 stored length
-#define SITE_WIDE 9 // BSG_ERR_WORKSPACE there: the factor wants the wide kernel
 #define REC_DONE (1ull << 63)
 #define REC_OFF(r) ((long long)(((r) >> 32) & 0x7fffffffull))
 #define REC_LEN(r) ((int)((r) & 0xffffull))

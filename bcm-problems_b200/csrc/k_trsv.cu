@@ -8,8 +8,8 @@
 //   backward y_i = dinv_u[i] * (x_i - sum_{k>i} U(i,k) y_k)
 //
 // mode 0 -- exact, sync-free: a warp solves one row, in level order within the
-//   block of consecutive rows its CTA owns, and each lane waits on the entry it
-//   needs.  "Solved" is encoded in the value itself: y is pre-filled with a NaN
+//   block of consecutive rows its CTA owns (or, where that does not pay, among all
+//   rows), and each lane waits on the entry it needs.  "Solved" is encoded in the value itself: y is pre-filled with a NaN
 //   bit pattern no arithmetic produces, and a 64-bit store publishes the result
 //   in one transaction.  A wait gives up (BSG_ERR_TIMEOUT) when globaltimer runs
 //   on for the limit without a row solved anywhere.
@@ -334,28 +334,6 @@ __global__ void k_trsv_sum(int n, const int *v, int *sum) {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	const int t = __reduce_add_sync(0xffffffffu, i < n ? v[i] : 0);
 	if ((threadIdx.x & 31) == 0 && t) atomicAdd(sum, t);
-}
-
-template <int G, typename VT>
-__global__ void __launch_bounds__(256) k_trsv_jacobi(int n, const int *__restrict__ rp, const int *__restrict__ ci,
-                                                     const VT *__restrict__ v, int skip_first,
-                                                     const double *__restrict__ dinv, const double *__restrict__ x,
-                                                     const double *__restrict__ yin, double *__restrict__ yout) {
-	const int lane32 = threadIdx.x & 31;
-	const int lane = lane32 & (G - 1);
-	const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	const int nwarps = (gridDim.x * blockDim.x) >> 5;
-	constexpr int RPW = 32 / G;
-	for (int r0 = warp * RPW; r0 < n; r0 += nwarps * RPW) {
-		int row = r0 + lane32 / G;
-		double s = 0.0;
-		if (row < n && yin) {
-			int b = rp[row] + skip_first, e = rp[row + 1];
-			for (int k = b + lane; k < e; k += G) s = fma((double)__ldcs(v + k), __ldg(yin + __ldcs(ci + k)), s);
-		}
-		s = group_sum<G>(s);
-		if (row < n && lane == 0) yout[row] = (x[row] - s) * dinv[row];
-	}
 }
 
 // y before an exact solve: nothing solved, no block claimed

@@ -668,7 +668,7 @@ def main():
                               "traffic_source": "profiles/k_sell_apply_heat128.md" if spmv_traffic else None,
                               "algorithmic_bytes": spmv_bytes, "ms_per_launch": t_spmv.value,
                               "peak_source": peak_kind},
-            "roofline_unet": {"bound": "tensor", "kernel": "U-Net forward (level 0: k_conv3_tc, tcgen05 + TMA; deeper levels: k_conv3t / k_conv3, mma.sync)",
+            "roofline_unet": {"bound": "tensor", "kernel": "U-Net forward (level 0: k_conv3_tc, tcgen05 + TMA; deeper levels: k_conv3t / k_conv3_few, mma.sync)",
                               "achieved": round(conv_tflops, 1), "peak": bf16_peak, "unit": "TFLOP/s",
                               "frac": round(conv_tflops / bf16_peak, 4), "ms_per_forward": round(t_unet, 4),
                               "flops": unet_flops(args.grid)},
