@@ -89,8 +89,9 @@ struct TrsvLimit {
 	unsigned t0 = 0, seen = 0; // in units of 1024 ns (registers are short here)
 	// whether to give up: another warp failed, or the limit has passed
 	__device__ __forceinline__ bool over(const unsigned *solved, int row, bsg_devstat *st) {
-		if (*(volatile int *)&st->code != 0) return true;
-		const unsigned now = (unsigned)(globaltimer_ns() >> 10) | 1u, cnt = *(const volatile unsigned *)solved;
+		const int code = *(volatile int *)&st->code; // (one round trip for both)
+		const unsigned cnt = *(const volatile unsigned *)solved, now = (unsigned)(globaltimer_ns() >> 10) | 1u;
+		if (code != 0) return true;
 		if (t0 == 0 || cnt != seen) {
 			t0 = now;
 			seen = cnt;
