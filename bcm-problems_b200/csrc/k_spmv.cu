@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256) k_interleave(int n, int nr, const double 
 // k_spmv_bsr3 for five or six vectors that lie side by side (k_interleave): there
 // a block's x is 18 contiguous doubles instead of six pieces of 24 bytes, one line
 // or two per block instead of six.  Bound of the strided form: the cache lines its
-// gathers touch (21 per 3 blocks; here about 14, values included).  Lane 9 t + 3 c
+// gathers touch (21 per 3 blocks; here 28.7 sectors, values included).  Lane 9 t + 3 c
 // + p holds block t of three, column c and the vectors 2 p and 2 p + 1 with their
 // three row sums, so that x comes in one 16-byte load and is used three times.  The
 // partial sums and the order they are added in are those of k_spmv_bsr3: the same

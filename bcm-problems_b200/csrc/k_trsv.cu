@@ -71,7 +71,7 @@ __global__ void k_scale_vec(int n, const double *x, const double *d, double *y) 
 // 7-point heat operator): 12^3 553 / 145, 32^3 1668 / 309, 47x40x33 3537 / 514,
 // 128^3 18690 / 5470; IC(0) 128^3 2075 / 1170; 2-D 500^2 22752 / 1836; a chain of
 // 100000 rows 437 / 21 ms (0.21 us a link).  Factors without locality go by rows
-// as before (k_trsv_rows, see trsv_scattered).
+// (k_trsv_rows, see trsv_scattered).
 #define TRSV_WARPS 32 // 24 warps: 47x40x33 580, 128^3 5520; 16: 760, 6600
 #define TRSV_M 2 // entries of a row each lane holds (32 TRSV_M a row; longer rows walk their head first)
 #define TRSV_ROWS_MAX 28000 // rows of a block: 8 bytes each in shared memory
